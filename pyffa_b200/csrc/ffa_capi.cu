@@ -3,6 +3,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <vector>
+
 #include "ffa_internal.cuh"
 
 using namespace ffa;
@@ -109,6 +111,110 @@ __global__ void mean_fi_kernel(const double *__restrict__ fi, int64_t n, double 
 
 unsigned blocks_for(int64_t n, int tb) { return (unsigned)((n + tb - 1) / tb); }
 
+// ------------------------------------------- one-dimensional field tables
+//
+// Taylor coefficients 0 .. N-1 of the logistic sigma(u0 + s x) in x, by the
+// recurrence of sigma' = sigma (1 - sigma):
+//   (n + 1) c_(n+1) = s (c_n - sum_i c_i c_(n-i)).
+constexpr int FL_SERIES = 12;
+
+void logistic_series(long double u0, long double s, long double c[FL_SERIES])
+{
+    c[0] = 1.0L / (1.0L + expl(-u0));
+    for (int n = 0; n + 1 < FL_SERIES; ++n) {
+        long double q = 0.0L;
+        for (int i = 0; i <= n; ++i) q += c[i] * c[n - i];
+        c[n + 1] = s * (c[n] - q) / (long double)(n + 1);
+    }
+}
+
+// Lowers a series on |x| <= 1/2 from FL_SERIES to 8 terms: each top term is
+// replaced by the lower powers of its Chebyshev polynomial T_n(2 x)
+// (Lanczos' economisation), which spreads its size / 2^(n-1) evenly over the
+// cell instead of leaving all of it at the edges.
+void economise(long double c[FL_SERIES])
+{
+    long double T[FL_SERIES][FL_SERIES] = {{0}};   // T_n(2 x), coefficient of x^a
+    T[0][0] = 1.0L;
+    T[1][1] = 2.0L;
+    for (int n = 2; n < FL_SERIES; ++n)
+        for (int a = 0; a <= n; ++a) T[n][a] = (a ? 4.0L * T[n - 1][a - 1] : 0.0L) - T[n - 2][a];
+    for (int n = FL_SERIES - 1; n >= 8; --n) {
+        const long double w = c[n] / T[n][n];
+        for (int a = 0; a <= n; ++a) c[a] -= w * T[n][a];
+    }
+}
+
+// The flutter and power tables of FieldK (formed in long double, stored as
+// double: flutter cells, then power entries).
+// Flutter cells: h = 2^-m with k h <= 0.04 for the sharpest fringe k = 16 / W:
+// the degree-7 fit then misses F by less than 1e-19 and F' by less than 1e-17
+// of k, below their rounding.  At most 2^17 cells (8 MB); a sharper fringe
+// (W below about 3e-3 of a 30 degree sector) keeps the sigmoids.
+// Power entries: spacing 2^-p with the first omitted binomial term below
+// 2^-57, over the map's radii and a quarter of their span on each side.
+void field_tables(FieldK &k, std::vector<double> &tab)
+{
+    double kmax = 0.0;
+    for (int j = 0; j < k.n_seg; ++j) kmax = fmax(kmax, fabs(k.seg_k[j]));
+    k.fl_n = 0;
+    if (kmax > 0.0 && isfinite(kmax)) {
+        int m = 0;
+        while (m < 40 && ldexp(kmax, -m) > 0.04) ++m;
+        const double cells = k.period * ldexp(1.0, m);
+        if (cells <= 131072.0) {
+            const int n = (int)ceil(cells);
+            k.fl_n = n + 2;
+            k.fl_scale = ldexp(1.0, m);
+            tab.resize(8 * (size_t)k.fl_n);
+            const long double h = ldexpl(1.0L, -m);
+            for (int j = 0; j < k.fl_n; ++j) {
+                const long double mid = ((long double)(j - 1) + 0.5L) * h;
+                long double sum[FL_SERIES] = {0};
+                for (int g = 0; g < k.n_seg; ++g) {
+                    const long double ks = k.seg_k[g];
+                    long double a[FL_SERIES], b[FL_SERIES];
+                    logistic_series(ks * (mid - (long double)k.seg_x0[g]), ks * h, a);
+                    logistic_series(-ks * (mid - (long double)k.seg_x1[g]), -ks * h, b);
+                    for (int n1 = 0; n1 < FL_SERIES; ++n1) {
+                        long double q = 0.0L;
+                        for (int i = 0; i <= n1; ++i) q += a[i] * b[n1 - i];
+                        sum[n1] += (long double)k.seg_y[g] * q;
+                    }
+                }
+                economise(sum);
+                for (int a = 0; a < 8; ++a) tab[8 * (size_t)j + a] = (double)sum[a];
+            }
+        }
+    }
+    k.pw_n = 0;
+    if (k.k != 0.0 && k.r_size > 1 && k.r_step > 0.0) {
+        const double span = k.r_step * (double)(k.r_size - 1);
+        const double lo = fmax(k.r_min - 0.25 * span, 0.25 * k.r_min), hi = k.r_min + 1.25 * span;
+        const double e = k.km1, c5 = fabs(e * (e - 1) * (e - 2) * (e - 3) * (e - 4) / 120.0);
+        if (lo > 0.0 && hi < 1e6) {
+            int p = 0;
+            while (p < 24 && c5 * pow(ldexp(0.5, -p) / lo, 5) > ldexp(1.0, -57)) ++p;
+            const double j0 = floor(lo * ldexp(1.0, p)), j1 = ceil(hi * ldexp(1.0, p));
+            if (j0 >= 1.0 && j1 - j0 < 65536.0 && j1 < 2147483647.0) {
+                k.pw_j0 = (int)j0;
+                k.pw_n = (int)(j1 - j0) + 1;
+                k.pw_scale = ldexp(1.0, p);
+                k.pw_h = ldexp(1.0, -p);
+                k.pw_c[0] = e;
+                k.pw_c[1] = e * (e - 1) / 2;
+                k.pw_c[2] = e * (e - 1) * (e - 2) / 6;
+                k.pw_c[3] = e * (e - 1) * (e - 2) * (e - 3) / 24;
+                for (int j = 0; j < k.pw_n; ++j) {
+                    const long double r = (long double)(k.pw_j0 + j) * (long double)k.pw_h;
+                    tab.push_back((double)((long double)k.B0 * powl(r, (long double)e)));
+                    tab.push_back((double)(1.0L / r));
+                }
+            }
+        }
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -171,28 +277,6 @@ int ffa_fieldmap_create(const ffa_field_desc *d, void *stream, ffa_fieldmap **ou
     k.inv_fi_step = d->fi_step > 0 ? 1.0 / d->fi_step : 0.0;
     k.c1 = d->k == 0.0 ? d->B0 : d->B0 * pow(k.r_ref, d->k - 1.0);
     k.kc1 = d->k * k.c1;
-    // binomial series of (1 + t)^(k-1) around the map centre (see FieldK)
-    k.pw_tlim = -1.0;
-    if (d->k != 0.0 && d->r_size > 1 && d->r_step > 0) {
-        const double m = d->k - 1.0;
-        k.pw_r0 = d->r_min + 0.5 * d->r_step * (double)(d->r_size - 1);
-        k.pw_inv_r0 = 1.0 / k.pw_r0;
-        k.pw_r0m = pow(k.pw_r0, m);
-        double c = 1.0;
-        for (int n = 0; n < 16; ++n) {
-            k.pw_c[n] = c;
-            c = c * (m - n) / (double)(n + 1);
-        }
-        // c is now the first omitted coefficient: largest |t| whose remainder
-        // bound |c| |t|^16 / (1 - |t|) stays below 2^-56 (1 - |t|)^m
-        double lo = 0.0, hi = 0.5;
-        for (int it = 0; it < 60; ++it) {
-            const double t = 0.5 * (lo + hi);
-            const double rem = fabs(c) * pow(t, 16) / (1.0 - t);
-            if (rem < ldexp(1.0, -56) * pow(1.0 - t, fabs(m))) lo = t; else hi = t;
-        }
-        k.pw_tlim = lo;
-    }
     k.B0f = (float)k.B0;
     k.c1f = (float)k.c1;
     k.kc1f = (float)k.kc1;
@@ -204,27 +288,32 @@ int ffa_fieldmap_create(const ffa_field_desc *d, void *stream, ffa_fieldmap **ou
         k.seg_yf[j] = (float)k.seg_y[j];
         k.seg_ykf[j] = (float)(k.seg_y[j] * k.seg_k[j]);
     }
-    for (int j = 0; j < d->n_convex; ++j) {
-        k.seg_yk[j] = k.seg_y[j] * k.seg_k[j];
-        const double hc = 0.5 * k.seg_k[j] * (k.seg_x1[j] - k.seg_x0[j]);
-        k.seg_hc[j] = hc <= 300.0 ? hc : 1e300;
-        k.seg_K[j] = hc <= 300.0 ? exp(-hc) : 0.0;
+    for (int j = 0; j < d->n_convex; ++j) k.seg_yk[j] = k.seg_y[j] * k.seg_k[j];
+    {
+        std::vector<double> tab;
+        field_tables(k, tab);
+        if (!tab.empty()) {
+            if (cudaMalloc(&fm->tables, sizeof(double) * tab.size()) != cudaSuccess) {
+                free(fm);
+                return FFA_ERR_NOMEM;
+            }
+            if (cudaMemcpy(fm->tables, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+                ffa_fieldmap_destroy(fm);
+                return FFA_ERR_CUDA;
+            }
+            k.fl_tab = fm->tables;
+            k.pw_tab = reinterpret_cast<const double2 *>(fm->tables + 8 * (size_t)k.fl_n);
+        }
     }
     if (d->max_order > 0) {
         const int64_t plane = d->r_size * d->fi_size;
-        if (cudaMalloc(&fm->nodes64, sizeof(double) * plane * k.npad) != cudaSuccess) {
-            free(fm);
-            return FFA_ERR_NOMEM;
-        }
-        if (cudaMalloc(&fm->nodes32, sizeof(float) * plane * k.npad) != cudaSuccess) {
-            cudaFree(fm->nodes64);
-            free(fm);
+        if (cudaMalloc(&fm->nodes64, sizeof(double) * plane * k.npad) != cudaSuccess ||
+            cudaMalloc(&fm->nodes32, sizeof(float) * plane * k.npad) != cudaSuccess) {
+            ffa_fieldmap_destroy(fm);
             return FFA_ERR_NOMEM;
         }
         if (launch_pack_nodes(*d, k.npad, fm->nodes64, fm->nodes32, as_stream(stream)) != cudaSuccess) {
-            cudaFree(fm->nodes64);
-            cudaFree(fm->nodes32);
-            free(fm);
+            ffa_fieldmap_destroy(fm);
             return FFA_ERR_CUDA;
         }
     }
@@ -263,6 +352,7 @@ int ffa_fieldmap_destroy(ffa_fieldmap *fm)
     if (!fm) return FFA_OK;
     if (fm->nodes64) cudaFree(fm->nodes64);
     if (fm->nodes32) cudaFree(fm->nodes32);
+    if (fm->tables) cudaFree(fm->tables);
     if (fm->harm) cudaFree(fm->harm);
     free(fm);
     return FFA_OK;

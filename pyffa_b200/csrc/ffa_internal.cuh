@@ -39,14 +39,20 @@ struct FieldK {
     double r_ref, inv_r_ref, inv_r_step, inv_fi_step;
     double c1, kc1;               // B0 r_ref^(k-1), k * c1
     double seg_yk[FFA_MAX_SEG];   // seg_y * seg_k
-    // paired sigmoids: half the edge-to-edge exponent c/2 = k (x1 - x0) / 2
-    // (a huge value disables the pairing) and exp(-c/2)
-    double seg_hc[FFA_MAX_SEG], seg_K[FFA_MAX_SEG];
-    // power law near the map centre: r^(k-1) = r0^(k-1) (1 + t)^(k-1),
-    // t = (r - r0) / r0, as a 16-term binomial series for |t| <= pw_tlim
-    // (truncation below 2^-56 relative); pw_tlim = -1 disables it
-    double pw_r0, pw_inv_r0, pw_tlim, pw_r0m;
-    double pw_c[16];
+    // Flutter table: F = sum_j y_j s1_j s2_j over one sector as degree-7
+    // polynomials (8 coefficients, lowest first, in x = q - j - 1/2,
+    // q = fs * fl_scale) over fl_n cells of 1 / fl_scale = 2^-m rad, a guard
+    // cell before and after the sector; fl_n = 0: no table
+    int32_t fl_n, pw_n;
+    double fl_scale;
+    const double *fl_tab;
+    // Power table: (B0 r_j^(k-1), 1 / r_j) at r_j = (pw_j0 + j) pw_h,
+    // pw_h = 1 / pw_scale = 2^-p m, and the binomial coefficients 1 .. 4 of
+    // the exponent k - 1; pw_n = 0: no table
+    int32_t pw_j0, pad3;
+    double pw_scale, pw_h;
+    const double2 *pw_tab;
+    double pw_c[4];
     // field-error harmonics: Bz += sum_k amp cos(m fi + phase) over the n_harm
     // rows (m, amp, phase, rmin, rmax) of the device table `harm` with
     // rmin <= r <= rmax (fi unwrapped)
@@ -111,6 +117,7 @@ struct ffa_fieldmap {
     ffa::FieldK k;
     double *nodes64;
     float *nodes32;
+    double *tables;       // device: flutter cells, then the power table
     double *harm;         // device, FFA_MAX_HARMONICS rows of 5
 };
 
