@@ -157,7 +157,10 @@ void field_tables(FieldK &k, std::vector<double> &tab)
 {
     double kmax = 0.0;
     for (int j = 0; j < k.n_seg; ++j) kmax = fmax(kmax, fabs(k.seg_k[j]));
-    k.fl_n = 0;
+    k.fl_n = 1;
+    k.fl_direct = 1;
+    k.fl_scale = 1.0;
+    tab.assign(8, 0.0);
     if (kmax > 0.0 && isfinite(kmax)) {
         int m = 0;
         while (m < 40 && ldexp(kmax, -m) > 0.04) ++m;
@@ -165,6 +168,7 @@ void field_tables(FieldK &k, std::vector<double> &tab)
         if (cells <= 131072.0) {
             const int n = (int)ceil(cells);
             k.fl_n = n + 2;
+            k.fl_direct = 0;
             k.fl_scale = ldexp(1.0, m);
             tab.resize(8 * (size_t)k.fl_n);
             const long double h = ldexpl(1.0L, -m);
@@ -187,7 +191,9 @@ void field_tables(FieldK &k, std::vector<double> &tab)
             }
         }
     }
-    k.pw_n = 0;
+    k.pw_n = 0;                                      // no r is inside: the entry is loaded, not used
+    k.pw_j0 = 0;
+    k.pw_scale = k.pw_h = 1.0;
     if (k.k != 0.0 && k.r_size > 1 && k.r_step > 0.0) {
         const double span = k.r_step * (double)(k.r_size - 1);
         const double lo = fmax(k.r_min - 0.25 * span, 0.25 * k.r_min), hi = k.r_min + 1.25 * span;
@@ -213,6 +219,7 @@ void field_tables(FieldK &k, std::vector<double> &tab)
             }
         }
     }
+    if (k.pw_n == 0) tab.insert(tab.end(), 2, 0.0);
 }
 
 }  // namespace
@@ -292,22 +299,24 @@ int ffa_fieldmap_create(const ffa_field_desc *d, void *stream, ffa_fieldmap **ou
     {
         std::vector<double> tab;
         field_tables(k, tab);
-        if (!tab.empty()) {
-            if (cudaMalloc(&fm->tables, sizeof(double) * tab.size()) != cudaSuccess) {
-                free(fm);
-                return FFA_ERR_NOMEM;
-            }
-            if (cudaMemcpy(fm->tables, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-                ffa_fieldmap_destroy(fm);
-                return FFA_ERR_CUDA;
-            }
-            k.fl_tab = fm->tables;
-            k.pw_tab = reinterpret_cast<const double2 *>(fm->tables + 8 * (size_t)k.fl_n);
+        k.unusual = k.fl_direct || k.k == 0.0;
+        if (cudaMalloc(&fm->tables, sizeof(double) * tab.size()) != cudaSuccess) {
+            free(fm);
+            return FFA_ERR_NOMEM;
         }
+        if (cudaMemcpy(fm->tables, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+            ffa_fieldmap_destroy(fm);
+            return FFA_ERR_CUDA;
+        }
+        k.fl_tab = fm->tables;
+        k.pw_tab = reinterpret_cast<const double2 *>(fm->tables + 8 * (size_t)k.fl_n);
     }
     if (d->max_order > 0) {
         const int64_t plane = d->r_size * d->fi_size;
-        if (cudaMalloc(&fm->nodes64, sizeof(double) * plane * k.npad) != cudaSuccess ||
+        int per = 0;
+        for (int a = 0; a < 12; a += 4) per += map_plane_width(d->max_order, a);
+        k.plane = plane;
+        if (cudaMalloc(&fm->nodes64, sizeof(double) * plane * per) != cudaSuccess ||
             cudaMalloc(&fm->nodes32, sizeof(float) * plane * k.npad) != cudaSuccess) {
             ffa_fieldmap_destroy(fm);
             return FFA_ERR_NOMEM;
@@ -434,7 +443,12 @@ static int push_impl(const ffa_fieldmap *fm, const ffa_rf_desc *rf, const ffa_ap
         p.rf.sp_phic = 0.5 * (rf->spiral_phi0 + p.rf.sp_phimax);
         memcpy(p.rf.gap_az, rf->gap_azimuth, sizeof(p.rf.gap_az));
     }
+    p.rf.single = rf->enable && !rf->spiral_nodes && !p.rf.physical_sum ? rf->ngaps - 1 : -1;
     p.ap = *ap;
+    if (!ap->enable) {
+        p.ap.rmin = p.ap.zmin = -INFINITY;
+        p.ap.rmax = p.ap.zmax = INFINITY;
+    }
     p.cs = *cs;
     p.st = *st;
     if (sc_step == 0) p.st.sc_pre = nullptr;
@@ -452,6 +466,7 @@ static int push_impl(const ffa_fieldmap *fm, const ffa_rf_desc *rf, const ffa_ap
         p.inv_cc = 1.0 / (c * c);
         p.inv_m = 1.0 / m;
         p.hqm = p.hq * p.inv_m;
+        p.inv_sc = sc_step > 0 ? 1.0 / (double)sc_step : 0.0;
     }
     p.status = status;
     if (xing) {

@@ -15,10 +15,21 @@ namespace ffa {
 
 constexpr double PI = 3.141592653589793;
 
+// Values per node in the plane of the float64 z-Taylor table that starts at
+// value a (0, 4, 8): four, or the one or two values left (three are padded)
+inline __host__ __device__ int map_plane_width(int max_order, int a)
+{
+    const int left = 3 * max_order - a;
+    return left >= 3 ? 4 : (left > 0 ? left : 0);
+}
+
 // Kernel-side view of the field (analytic parameters precomputed once and the
-// packed z-Taylor node table).  Node (i, j) of the r x fi grid holds, for
-// n = 1..max_order, (bz_n, bfi_n, br_n), padded to `npad` values so a node is
-// 32 B (float32) or 64 B (float64) aligned for max_order <= 2.
+// packed z-Taylor table).  A node (i, j) of the r x fi grid has, for
+// n = 1..max_order, the values (bz_n, bfi_n, br_n).  The float32 table keeps a
+// node's values together, padded to `npad` (4, 8, 12).  The float64 table is
+// split into planes of up to four values per node (map_plane_width), each
+// over all nodes: value a + b of a node, a = 0, 4, 8, is at
+// a * plane + node * width + b with `plane` the number of nodes.
 struct FieldK {
     int32_t nsectors, n_spoly, n_spolyp, n_seg, max_order, npad;
     double B0, k, km1, B0k;       // B0, k, k - 1, B0 * k
@@ -30,7 +41,7 @@ struct FieldK {
     double seg_k[FFA_MAX_SEG];    // 16 / W0
     double seg_y[FFA_MAX_SEG];    // y02 * |y01|
     double r_min, r_step, fi_min, fi_step;
-    int64_t r_size, fi_size;
+    int64_t r_size, fi_size, plane;
     const double *nodes64;
     const float *nodes32;
     // float32 field: B0 r^(k-1) = c1 * (1 + eps)^(k-1), eps = (r - r_ref) / r_ref
@@ -42,14 +53,16 @@ struct FieldK {
     // Flutter table: F = sum_j y_j s1_j s2_j over one sector as degree-7
     // polynomials (8 coefficients, lowest first, in x = q - j - 1/2,
     // q = fs * fl_scale) over fl_n cells of 1 / fl_scale = 2^-m rad, a guard
-    // cell before and after the sector; fl_n = 0: no table
-    int32_t fl_n, pw_n;
+    // cell before and after the sector; fl_direct: no table (one dummy cell),
+    // the sigmoids are evaluated
+    int32_t fl_n, fl_direct;
+    int32_t unusual, pad3;   // fl_direct, or k == 0
     double fl_scale;
     const double *fl_tab;
     // Power table: (B0 r_j^(k-1), 1 / r_j) at r_j = (pw_j0 + j) pw_h,
     // pw_h = 1 / pw_scale = 2^-p m, and the binomial coefficients 1 .. 4 of
-    // the exponent k - 1; pw_n = 0: no table
-    int32_t pw_j0, pad3;
+    // the exponent k - 1; without a table one dummy entry that no r reaches
+    int32_t pw_j0, pw_n;
     double pw_scale, pw_h;
     const double2 *pw_tab;
     double pw_c[4];
@@ -64,7 +77,8 @@ struct FieldK {
 };
 
 struct RFK {
-    int32_t enable, ngaps, physical_sum, pad0;
+    int32_t enable, ngaps, physical_sum;
+    int32_t single;       // the one fixed gap that acts (the last), -1: none, or spiral gaps or the sum of all
     double poly_x[FFA_MAX_GAPS][4];
     double poly_y[FFA_MAX_GAPS][4];
     double box[FFA_MAX_GAPS][4];
@@ -104,6 +118,7 @@ struct PushK {
     double inv_m;       // 1 / m
     double inv_cc;      // 1 / c^2
     double inv_mmcc;    // 1 / (m^2 c^2)
+    double inv_sc;      // 1 / sc_step (0 without space charge)
 };
 
 inline __host__ __device__ bool xing_on(const PushK &p)

@@ -40,6 +40,11 @@ __device__ __forceinline__ void ldg_v4(const double *p, double t[4])
         : "=d"(t[0]), "=d"(t[1]), "=d"(t[2]), "=d"(t[3]) : "l"(p));
 }
 
+__device__ __forceinline__ void ldg_v2(const double *p, double t[2])
+{
+    asm("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(t[0]), "=d"(t[1]) : "l"(p));
+}
+
 __device__ __forceinline__ void ldg_v8(const float *p, float t[8])
 {
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -52,6 +57,28 @@ __device__ __forceinline__ void ldg_v8(const float *p, float t[8])
 // integers 0 .. 2^32 - 1)
 constexpr double INT_MAGIC = 6755399441055744.0;
 constexpr int INT_HI = 0x43380000;
+
+// x^(-1/2) and 1 / x for normal positive x, without a branch: the hardware's
+// approximation (relative error about 2^-20, PTX ISA rsqrt.approx / rcp.approx)
+// refined by one third-order Householder step.  With e = 1 - x y^2 (or 1 - x y)
+// the series of (1 - e)^(-1/2) (or 1 / (1 - e)) to e^2 leaves 5/16 e^3 (e^3),
+// below 2^-58, so the result is right to about an ulp.  The library functions
+// add range tests whose branches keep a step's chains from overlapping.
+__device__ __forceinline__ double rsqrt64(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+__device__ __forceinline__ double rcp64(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
 
 // Flutter sum and its azimuth derivative from the magnets' sigmoids, for
 // lattices without a flutter table (fringes sharper than the table's limit).
@@ -94,68 +121,74 @@ __device__ __noinline__ double power_direct(const FieldK &f, double r) { return 
 // latency and issue.  Measured (720 steps, z-Taylor order 2, RF): 1e5
 // particles Boris 2.47 -> 2.07 ms, RK4 11.3 -> 9.6 ms; 1e4 particles, order 4:
 // 1.87 -> 1.74 ms; 1280 azimuth-domain tracks of 523 steps: 2.46 -> 1.59 ms.
-__device__ __forceinline__ void analytic_b64(const FieldK &f, double ri, double ir, double fim, double zi,
-                                             double &Bz, double &Br, double &Bfi)
+struct Tables {
+    double c[8], x;      // flutter cell and the position in it
+    double2 e;           // power entry (B0 r_j^(k-1), 1 / r_j)
+    double d;            // r - r_j
+    double fs, spiral_p;
+    bool pw;             // r is inside the power table
+};
+
+// The table entries of a point, loaded unconditionally (a map without a table
+// has one dummy entry), so that these loads and the map's are in flight
+// together.
+__device__ __forceinline__ Tables tables_fetch(const FieldK &f, double ri, double fim)
 {
     // theta' = (fi mod P) - s(r), reduced mod P again.  Without a spiral
     // (all-zero coefficients evaluate to exactly 0) the callers' fim is
     // reduced already: the second reduction would only map a fim within an
     // ulp of P to about 0 (a step lands there with probability ~1e-16), so
     // it is skipped with the polynomials.
-    double spiral_p = 0.0;
-    double fs = fim;
+    Tables t;
+    t.spiral_p = 0.0;
+    t.fs = fim;
     if (!f.spiral_zero) {
         double spiral = 0.0;
         for (int a = 0; a < f.n_spoly; ++a) spiral = spiral * ri + f.spoly[a];
-        for (int a = 0; a < f.n_spolyp; ++a) spiral_p = spiral_p * ri + f.spolyp[a];
-        fs = fim - spiral;
-        fs -= f.period * floor(fs * f.inv_period);
+        for (int a = 0; a < f.n_spolyp; ++a) t.spiral_p = t.spiral_p * ri + f.spolyp[a];
+        t.fs = fim - spiral;
+        t.fs -= f.period * floor(t.fs * f.inv_period);
     }
-    double F, Fp;
-    if (f.fl_n > 0) {
-        // cell j covers [j, j + 1) cells of azimuth; one guard cell on each
-        // side takes a reduction that rounded just outside the sector
-        const double q = fma(fs, f.fl_scale, -0.5), qi = q + INT_MAGIC;
-        const int j = min(max(__double2loint(qi) + 1, 0), f.fl_n - 1);
-        const double x = q - (qi - INT_MAGIC);
-        double c[8];
-        ldg_v4(f.fl_tab + 8 * j, c);
-        ldg_v4(f.fl_tab + 8 * j + 4, c + 4);
-        F = c[7];
-        Fp = 0.0;
+    // cell j covers [j, j + 1) cells of azimuth; one guard cell on each side
+    // takes a reduction that rounded just outside the sector
+    const double q = fma(t.fs, f.fl_scale, -0.5), qi = q + INT_MAGIC;
+    const int j = min(max(__double2loint(qi) + 1, 0), f.fl_n - 1);
+    t.x = q - (qi - INT_MAGIC);
+    ldg_v4(f.fl_tab + 8 * j, t.c);
+    ldg_v4(f.fl_tab + 8 * j + 4, t.c + 4);
+    const double pi = fma(ri, f.pw_scale, INT_MAGIC);
+    const int k = __double2loint(pi) - f.pw_j0;
+    t.pw = __double2hiint(pi) == INT_HI && (unsigned)k < (unsigned)f.pw_n;
+    t.d = fma(INT_MAGIC - pi, f.pw_h, ri);
+    t.e = __ldg(f.pw_tab + (t.pw ? k : 0));
+    return t;
+}
+
+// F, F', B0 r^(k-1) and its k-fold from the entries of a point
+__device__ __forceinline__ void tables_eval(const FieldK &f, const Tables &t, double ri, double &F, double &Fp,
+                                            double &G, double &kG)
+{
+    F = t.c[7];
+    Fp = 0.0;
 #pragma unroll
-        for (int a = 6; a >= 0; --a) {
-            Fp = (a == 6) ? F : fma(Fp, x, F);
-            F = fma(F, x, c[a]);
-        }
-        Fp *= f.fl_scale;
-    } else {
-        const double2 v = flutter_direct(f, fs);
-        F = v.x;
-        Fp = v.y;
+    for (int a = 6; a >= 0; --a) {
+        Fp = (a == 6) ? F : fma(Fp, t.x, F);
+        F = fma(F, t.x, t.c[a]);
     }
-    double B0r, B0r_p;
-    if (f.k == 0.0) {
-        B0r = f.B0;
-        B0r_p = 0.0;
-    } else {
-        const double qi = fma(ri, f.pw_scale, INT_MAGIC);
-        const int j = __double2loint(qi) - f.pw_j0;
-        double G;
-        if (__double2hiint(qi) == INT_HI && (unsigned)j < (unsigned)f.pw_n) {
-            const double2 e = __ldg(f.pw_tab + j);      // B0 r_j^(k-1), 1 / r_j
-            const double t = fma(INT_MAGIC - qi, f.pw_h, ri) * e.y;
-            const double P = fma(t, fma(t, fma(t, f.pw_c[3], f.pw_c[2]), f.pw_c[1]), f.pw_c[0]);
-            G = fma(e.x * t, P, e.x);
-        } else {
-            G = power_direct(f, ri);
+    Fp *= f.fl_scale;
+    const double u = t.d * t.e.y;
+    const double P = fma(u, fma(u, fma(u, f.pw_c[3], f.pw_c[2]), f.pw_c[1]), f.pw_c[0]);
+    G = fma(t.e.x * u, P, t.e.x);
+    if (!t.pw) G = power_direct(f, ri);
+    kG = f.k * G;
+    if (f.unusual) {                     // no flutter table, or a field index of 0
+        if (f.fl_direct) {
+            const double2 v = flutter_direct(f, t.fs);
+            F = v.x;
+            Fp = v.y;
         }
-        B0r_p = f.k * G;
-        B0r = G * ri;
+        if (f.k == 0.0) G = f.B0 / ri;
     }
-    Bz = B0r * F;
-    Bfi = B0r * Fp * ir * zi;    // ir = 1 / ri to an ulp
-    Br = (B0r_p * F - B0r * Fp * spiral_p) * zi;
 }
 
 // Bilinear lookup of the z-Taylor coefficients: int() truncation, index
@@ -165,9 +198,13 @@ __device__ __forceinline__ void analytic_b64(const FieldK &f, double ri, double 
 // clamp applies anyway, and a NaN coordinate truncates to node 0.
 __device__ __forceinline__ int trunc_index(double q) { return __double2int_rz(q); }
 
-template <int MAXO>
-__device__ __forceinline__ void high_order_b64(const FieldK &f, double x, double y, double z,
-                                               double &Bz, double &Bfi, double &Br, int &clamped)
+// The cell of (x, y) in the z-Taylor map and the position in it
+struct Cell {
+    int node;            // i * fi_size + j
+    double tx, ty;
+};
+
+__device__ __forceinline__ Cell map_cell(const FieldK &f, double x, double y, int &clamped)
 {
     // cell index and weights from (x - x_min) times 1 / step: within an ulp
     // of the reference's quotient; where that moves the index across a node
@@ -176,50 +213,89 @@ __device__ __forceinline__ void high_order_b64(const FieldK &f, double x, double
     const double qx = (x - f.r_min) * f.inv_r_step;
     const double qy = (y - f.fi_min) * f.inv_fi_step;
     const int nr = (int)f.r_size, nf = (int)f.fi_size;
-    int i = trunc_index(qx);
-    int j = trunc_index(qy);
-    if (i < 0) { i = 0; ++clamped; }
-    else if (i >= nr - 1) { i = nr - 2; ++clamped; }
-    if (j < 0) { j = 0; ++clamped; }
-    else if (j >= nf - 1) { j = nf - 2; ++clamped; }
-    const double tx = qx - (double)i;
-    const double ty = qy - (double)j;
-    const double w00 = (1.0 - tx) * (1.0 - ty), w01 = (1.0 - tx) * ty;
-    const double w10 = tx * (1.0 - ty), w11 = tx * ty;
-    constexpr int NP = (3 * MAXO <= 4) ? 4 : ((3 * MAXO <= 8) ? 8 : 12);
+    const int i0 = trunc_index(qx), j0 = trunc_index(qy);
+    const int i = min(max(i0, 0), nr - 2), j = min(max(j0, 0), nf - 2);
+    clamped += (i != i0) + (j != j0);
+    return {i * nf + j, qx - (double)i, qy - (double)j};
+}
+
+// The sums of the z-Taylor terms: hz = sum_n bz_n z^(2n), and hf, hr =
+// sum_n (bfi_n, br_n) z^(2n), which the caller multiplies by z.
+//
+// A warp load costs the L1 data pipe one cycle per distinct 128-byte line it
+// touches, and at least its bytes / 128 (measured: 8.5 cycles for a 32-byte load
+// of one line, 16 for 16 lines, 32 for 32), and large bunches are bound by
+// that pipe.  So the table is split into planes of one load each (FieldK):
+// four nodes of a row share a line, where whole 64-byte nodes put two loads
+// on every line of two.  Order 2, 1e5 particles, 720 steps: 1.74 ms with whole
+// nodes, 1.54 ms in planes; 1e6 particles, 60 steps with space charge (128
+// registers): 1.90 and 1.69 ms.
+template <int MAXO>
+__device__ __forceinline__ void z_taylor64(const FieldK &f, const Cell &cell, double z, double &hz, double &hf,
+                                           double &hr)
+{
     constexpr int NV = 3 * MAXO;
-    const double *nd[4];
-    nd[0] = f.nodes64 + (i * nf + j) * NP;    // (i, j)
-    nd[1] = nd[0] + NP;                       // (i, j+1)
-    nd[2] = nd[0] + nf * NP;                  // (i+1, j)
-    nd[3] = nd[2] + NP;                       // (i+1, j+1)
-    const double w[4] = {w00, w01, w10, w11};
-    // accumulate node by node in the reference's order w00, w01, w10, w11;
-    // a node (32, 64 or 96 B) is read in 32-byte loads: half the load
-    // instructions of 16-byte pairs, and the L1 throughput they take is the
-    // kernel's bound
-    double acc[NV > 0 ? NV : 1];
+    const double tx = cell.tx, ty = cell.ty;
+    const double w[4] = {(1.0 - tx) * (1.0 - ty), (1.0 - tx) * ty, tx * (1.0 - ty), tx * ty};
+    const int nf = (int)f.fi_size;
+    // accumulate node by node in the reference's order w00, w01, w10, w11
+    double acc[NV];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int a = 0; a < NV; a += 4) {
+        constexpr int LAST = NV % 4 == 3 ? 4 : NV % 4;
+        const int W = NV - a >= 4 || LAST == 0 ? 4 : LAST;
+        const double *pl = f.nodes64 + a * f.plane + (int64_t)cell.node * W;
+        const double *nd[4] = {pl, pl + W, pl + nf * W, pl + nf * W + W};
 #pragma unroll
-        for (int a = 0; a < NV; a += 4) {
+        for (int k = 0; k < 4; ++k) {
             double t[4];
-            ldg_v4(nd[k] + a, t);
+            if (W == 4) ldg_v4(nd[k], t);
+            else if (W == 2) ldg_v2(nd[k], t);
+            else t[0] = __ldg(nd[k]);
 #pragma unroll
-            for (int b = 0; b < 4; ++b)
+            for (int b = 0; b < W; ++b)
                 if (a + b < NV) acc[a + b] = (k == 0) ? w[0] * t[b] : acc[a + b] + w[k] * t[b];
         }
     }
     const double z2 = z * z;
-    double ze = z2, zo = ze * z;
+    hz = acc[NV - 3];
+    hf = acc[NV - 2];
+    hr = acc[NV - 1];
 #pragma unroll
-    for (int n = 0; n < MAXO; ++n) {
-        Bz += acc[3 * n] * ze;
-        Bfi += acc[3 * n + 1] * zo;
-        Br += acc[3 * n + 2] * zo;
-        ze *= z2;
-        zo *= z2;
+    for (int n = MAXO - 2; n >= 0; --n) {
+        hz = fma(hz, z2, acc[3 * n]);
+        hf = fma(hf, z2, acc[3 * n + 1]);
+        hr = fma(hr, z2, acc[3 * n + 2]);
     }
+    hz *= z2;
+    hf *= z2;
+    hr *= z2;
+}
+
+// The field at (r, fim, z): the mid-plane field with its z-linear terms from
+// the two one-dimensional tables, and the z-Taylor terms from the map.  ir =
+// 1 / r to an ulp.  The cell coordinates of the tables are exact (power-of-two
+// cells), so their evaluation adds a few ulp, as the exponentials and the
+// 16-term series about the map centre did before; without their branches and
+// divisions, and with every load issued before the first use, the field is one
+// stretch of code whose chains overlap.  Measured (720 steps, z-Taylor order 2,
+// RF): 1e5 particles Boris 2.47 -> 2.07 ms, RK4 11.3 -> 9.6 ms; 1280
+// azimuth-domain tracks of 523 steps: 2.46 -> 1.43 ms.
+template <int MAXO>
+__device__ __forceinline__ void field64(const FieldK &f, double r, double ir, double fim, double z, double &Bz,
+                                        double &Br, double &Bfi, int &clamped)
+{
+    double hz = 0.0, hf = 0.0, hr = 0.0;
+    Cell cell;
+    if constexpr (MAXO >= 1) cell = map_cell(f, r, fim, clamped);
+    const Tables t = tables_fetch(f, r, fim);
+    if constexpr (MAXO >= 1) z_taylor64<MAXO>(f, cell, z, hz, hf, hr);
+    double F, Fp, G, kG;
+    tables_eval(f, t, r, F, Fp, G, kG);
+    const double B0r = G * r, B0Fp = B0r * Fp;
+    Bz = fma(B0r, F, hz);
+    Bfi = fma(B0Fp, ir, hf) * z;
+    Br = (fma(kG, F, hr) - B0Fp * t.spiral_p) * z;
 }
 
 // bharmonics_kernel_1d (src/FFAG_Field.py:1541-1587) for one particle: the
@@ -306,6 +382,19 @@ __device__ __forceinline__ double3 rf_spiral64(const RFK &rf, double acc, double
     return make_double3((acc * er) * s, ((acc * ez) * z) * s, (acc * ef) * s);   // Er, Ez, Efi
 }
 
+// Er, Efi of fixed gap g at a particle inside its angular window (out of
+// line: a few steps of a turn come here)
+__device__ __noinline__ double2 gap_field64(const RFK &rf, int g, double acc, double r, double fi, double rfph)
+{
+    double sf, cf;
+    sincos(fi, &sf, &cf);
+    if (!gap_inside(rf, g, r * cf, r * sf)) return make_double2(0.0, 0.0);
+    double sd, cd;
+    sincos(rf.theta_n[g] - fi, &sd, &cd);
+    const double s = sin(rfph + rf.rf_shift[g]);
+    return make_double2((acc * cd) * s, (acc * sd) * s);
+}
+
 // RF field (cylindrical r, z, fi components) times sin(RF phase +
 // rf_shift[gap]).  Fixed gaps, reference semantics: every gap's emap_kernel
 // call overwrites the field, so only the last gap contributes (no Ez);
@@ -327,34 +416,64 @@ __device__ __forceinline__ void rf_field64(const RFK &rf, double acc, double r, 
     const int g0 = rf.physical_sum ? 0 : rf.ngaps - 1;
     for (int g = g0; g < rf.ngaps; ++g) {
         if (!in_window(rf, g, fi)) continue;
-        double sf, cf;
-        sincos(fi, &sf, &cf);
-        if (!gap_inside(rf, g, r * cf, r * sf)) continue;
-        double sd, cd;
-        sincos(rf.theta_n[g] - fi, &sd, &cd);
-        const double s = sin(rfph + rf.rf_shift[g]);
-        Er += (acc * cd) * s;
-        Efi += (acc * sd) * s;
+        const double2 e = gap_field64(rf, g, acc, r, fi, rfph);
+        Er += e.x;
+        Efi += e.y;
     }
+}
+
+// The RF field of the FP64 kernels at a point: false (and no field) outside
+// the gaps.  With the reference's semantics on fixed gaps (rf.single >= 0,
+// the one gap that acts) the angular window decides inline and only the few
+// steps inside it call gap_field64.
+__device__ __noinline__ double3 rf_general64(const RFK &rf, double acc, double r, double fi, double z, double rfph)
+{
+    double Er, Ez, Efi;
+    rf_field64(rf, acc, r, fi, z, rfph, Er, Ez, Efi);
+    return make_double3(Er, Ez, Efi);
+}
+
+__device__ __forceinline__ bool rf_hit64(const RFK &rf, const double *acc, double r, double fi, double z, double rfph,
+                                         double3 &e)
+{
+    if (rf.single >= 0) {
+        if (!in_window(rf, rf.single, fi)) return false;
+        const double2 g = gap_field64(rf, rf.single, __ldg(acc), r, fi, rfph);
+        e = make_double3(g.x, 0.0, g.y);
+        return g.x != 0.0 || g.y != 0.0;
+    }
+    if (!rf.enable) return false;
+    e = rf_general64(rf, __ldg(acc), r, fi, z, rfph);
+    return e.x != 0.0 || e.y != 0.0 || e.z != 0.0;
+}
+
+__device__ __noinline__ double3 wide_rotation(double y, double x)
+{
+    const double a = atan2(y, x);
+    double s, c;
+    sincos(a, &s, &c);
+    return make_double3(a, s, c);
 }
 
 // Azimuth change of one step and its sine / cosine, from the new position's
 // unit vector in the local frame: sin and cos of the step angle are y / r and
 // x / r (r^-1 is at hand from the drift); a step turns the particle by about
 // 2 pi / (steps per turn), and for |sin| < 0.02 the angle is the arcsine series
-//   asin(s) = s (1 + s^2/6 + 3 s^4/40 + 5 s^6/112 + 35 s^8/1152 + 63 s^10/2816)
-// (truncation < 1e-22 relative): no division and no sin/cos series.
+//   asin(s) = s (1 + s^2/6 + 3 s^4/40 + 5 s^6/112 + 35 s^8/1152)
+// (truncation < 3e-19 relative): no division and no sin/cos series.
 __device__ __forceinline__ void step_rotation(double y, double x, double ir, double &a, double &s, double &c)
 {
     const double s0 = y * ir;
     if (x > 0.0 && fabs(s0) < 0.02) {
         const double s2 = s0 * s0;
-        a = s0 * (1.0 + s2 * (1.0 / 6 + s2 * (3.0 / 40 + s2 * (5.0 / 112 + s2 * (35.0 / 1152 + s2 * (63.0 / 2816))))));
+        a = s0 * (1.0 + s2 * (1.0 / 6 + s2 * (3.0 / 40 + s2 * (5.0 / 112 + s2 * (35.0 / 1152)))));
         s = s0;
         c = x * ir;
     } else {
-        a = atan2(y, x);
-        sincos(a, &s, &c);
+        const double3 w = wide_rotation(y, x);
+        a = w.x;
+        s = w.y;
+        c = w.z;
     }
 }
 
@@ -496,6 +615,12 @@ __device__ __forceinline__ void xing_check(const ffa_crossing &xc, int64_t i, in
     }
 }
 
+// Position of step gs in its space-charge interval (0 in the first interval)
+__device__ __forceinline__ int sc_phase(const PushK &p, int64_t gs)
+{
+    return gs >= p.sc_step ? (int)(gs % p.sc_step) : 0;
+}
+
 // Linear extrapolation of the space-charge field between updates
 // (src/FFAG_track.py:449-478).
 struct SCExtrap {
@@ -510,10 +635,11 @@ struct SCExtrap {
             if (pp) { eqr = S.e_pp_r[i]; eqz = S.e_pp_z[i]; eqf = S.e_pp_fi[i]; }
         }
     }
-    __device__ void apply(int64_t gs, int sc_step, double &esr, double &esz, double &esf) const
+    // ph: the step's position gs mod sc_step in its interval (0 in the first)
+    __device__ void apply(int ph, double inv_sc, double &esr, double &esz, double &esf) const
     {
         if (!pre) return;
-        const double sf = gs >= sc_step ? (double)(gs % sc_step) / (double)sc_step : 0.0;
+        const double sf = (double)ph * inv_sc;
         if (pp) {
             esr = epr + sf * (epr - eqr);
             esz = epz + sf * (epz - eqz);
@@ -635,21 +761,197 @@ __device__ __forceinline__ void field_mixed(const FieldK &f, double r, double ir
 
 // ------------------------------------------------------------ Boris fp64
 
-// One-warp blocks, at most 80 registers.  The register file is split over
+// One-warp blocks; at 80 registers a launch holds the most warps that run
+// without heavy spills.  The register file is split over
 // the SM's four schedulers (16384 registers each): 80 x 32 = 2560 registers
 // per warp gives 6 warps per scheduler, 24 per SM, 3552 on 148 SMs, so the
 // 3125 warps of a 1e5-particle bunch are resident in one wave.  At 88
 // registers it is 5 per scheduler (2960 warps): the last 165 warps then run
 // all their steps as a second, nearly empty wave (measured: 5.09 ms per
 // 720-step turn at 88 registers, 3.81 ms at 80).
-constexpr int BORIS_TB = 32;
 
-// NREG: the register cap.  80 is the default launch shape; the compensated
+// The FP64 step carries u = gamma v and 1 / gamma instead of the velocities.
+// The reference forms gamma from |v| at the start of every step and again
+// after each half kick; but a step without an electric field turns u and
+// leaves gamma as it is, and u is known from the step before.  So a
+// particle's 1 / gamma is recomputed only after a kick (an RF gap, space
+// charge); the velocities are formed where they are read: at the end of the
+// launch, at a crossing, and when a particle leaves flight (not injected or
+// lost particles keep velocities, which the reference's Cartesian round trip
+// perturbs).  A live step is then one stretch of code without branches but the
+// rare ones (gap window, wide steps), so its independent chains overlap.
+// Large bunches are bound by the L1 data pipe (z_taylor64), small ones by one
+// step's chain: the node loads from L2 (about 300 cycles) and some 110
+// dependent FP64 operations of 8 cycles.  720 steps, with the tables of field64
+// and the planes of z_taylor64: 1e5 particles, order 2, RF 2.47 -> 1.54 ms; 1e4
+// particles, order 4, 1.88 -> 0.79 ms; 1e6 particles, 60 steps with space
+// charge 2.05 -> 1.69 ms.
+template <int MAXO, bool SC, bool XING, int NREG, bool HARM = false>
+__global__ void __maxnreg__(NREG) boris_f64_kernel(const __grid_constant__ PushK p)
+{
+    const int64_t t_ = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t_ >= p.n) return;
+    const int64_t i = p.st.order ? (int64_t)__ldg(p.st.order + t_) : t_;   // the particle this thread advances
+    const FieldK &f = p.f;
+    const ffa_state_soa &S = p.st;
+    // (a, b, c): in flight u_r, u_fi, u_z; otherwise vr, dfi/dt, vz
+    double r = S.r[i], a = S.vr[i], z = S.z[i], c = S.vz[i], fi = S.fi[i], b = S.f5[i];
+    double rfph = S.rf[i];
+    int inj = S.inj[i], surv = S.surv[i];
+    // the launch's step at which the particle is injected (none: -1)
+    const int64_t injs = (S.inj_step ? (int64_t)S.inj_step[i] : -1) - p.step0;
+    const int inj_at = injs >= 0 && injs < p.nsteps ? (int)injs : -1;
+    double esr = S.esc_r[i], esz = S.esc_z[i], esf = S.esc_fi[i];
+    const bool esc = SC || esr != 0.0 || esz != 0.0 || esf != 0.0;   // also for NaN
+    SCExtrap ex;
+    int ph = 0;
+    if (SC) {
+        ex.load(S, i);
+        ph = sc_phase(p, p.step0);
+    }
+    double ir = 1.0 / r, ig = 0.0;           // 1 / r and 1 / gamma, carried
+    auto take_off = [&]() {
+        const double vf = r * b, x = 1 - (a * a + vf * vf + c * c) * p.inv_cc, g = rsqrt(x);
+        a *= g;
+        b = g * vf;
+        c *= g;
+        ig = x * g;
+    };
+    auto land = [&]() {
+        a *= ig;
+        b = r > 1e-12 ? b * ig * ir : 0.0;
+        c *= ig;
+    };
+    // the turn of u about -B by the angle of the step (Boris)
+    auto turn = [&](double Bz, double Br, double Bfi) {
+        const double cb = -p.hqm * ig;
+        const double tx = cb * Br, ty = cb * Bfi, tz = cb * Bz;
+        const double pa = a + (b * tz - c * ty);
+        const double pb = b + (c * tx - a * tz);
+        const double pc = c + (a * ty - b * tx);
+        const double sb = 2.0 * rcp64(1.0 + (tx * tx + ty * ty + tz * tz));
+        const double sx = sb * tx, sy = sb * ty, sz = sb * tz;
+        a += (pb * sz - pc * sy);
+        b += (pc * sx - pa * sz);
+        c += (pa * sy - pb * sx);
+    };
+    auto kick = [&](const double3 &e) {      // half the step's electric kick (e: r, z, fi)
+        a = fma(p.hqm, e.x, a);
+        b = fma(p.hqm, e.z, b);
+        c = fma(p.hqm, e.y, c);
+        ig = rsqrt64(fma(a * a + b * b + c * c, p.inv_cc, 1.0));
+    };
+    bool live = inj == 1 && surv == 1;
+    if (live) take_off();
+    int lost = 0, oob = 0;
+    const double *drf = p.drf + p.step0;
+
+    for (int s = 0; s < p.nsteps; ++s) {
+        if (s == inj_at) {
+            inj = 1;
+            surv = 1;
+            if (!live) take_off();
+            live = true;
+        }
+        if (SC) {
+            ex.apply(ph, p.inv_sc, esr, esz, esf);
+            const int64_t gs = p.step0 + s;
+            ph = (gs + 1 <= p.sc_step || ph + 1 == p.sc_step) ? 0 : ph + 1;   // sc_phase of the next step
+        }
+        double pre[7];
+        const int surv0 = surv;
+        if constexpr (XING) {
+            pre[0] = r; pre[2] = z; pre[4] = fi; pre[6] = rfph;
+            pre[1] = live ? a * ig : a;
+            pre[3] = live ? c * ig : c;
+            pre[5] = live ? (r > 1e-12 ? b * ig * ir : 0.0) : b;
+        }
+        if (live) {
+            // fi mod the sector; a multiply by 1 / period instead of the
+            // division can move floor() only where fi / period is within an
+            // ulp of an integer, i.e. between two equal values of the
+            // periodic field (0 and the period)
+            const double fim = fi - f.period * floor(fi * f.inv_period);
+            double Bz, Br, Bfi;
+            field64<MAXO>(f, r, ir, fim, z, Bz, Br, Bfi, oob);
+            if constexpr (HARM) Bz += harmonics_bz(f.harm, f.n_harm, r, fi);
+            if (r > p.ap.rmax || r < p.ap.rmin || z > p.ap.zmax || z < p.ap.zmin) {   // infinite when off
+                surv = 0;
+                ++lost;
+            }
+            double3 e = make_double3(0.0, 0.0, 0.0);
+            const bool hit = rf_hit64(p.rf, p.acc + p.step0 + s, r, fi, z, rfph, e);
+            if (esc || hit) {
+                if (esc) {
+                    if (!SC) { esr = S.esc_r[i]; esz = S.esc_z[i]; esf = S.esc_fi[i]; }   // not held over the loop
+                    e.x += esr;
+                    e.y += esz;
+                    e.z += esf;
+                }
+                kick(e);
+                turn(Bz, Br, Bfi);
+                kick(e);
+            } else {
+                turn(Bz, Br, Bfi);
+            }
+            // drift, in the frame x along r-hat, y along fi-hat
+            const double dtg = p.dt * ig;
+            const double xn = fma(a, dtg, r), yn = b * dtg;
+            z = fma(c, dtg, z);
+            const double rr2 = xn * xn + yn * yn;
+            ir = rsqrt64(rr2);
+            r = rr2 * ir;
+            double dfi, sn, cn;
+            step_rotation(yn, xn, ir, dfi, sn, cn);
+            fi = fi + dfi;
+            const double an = a * cn + b * sn;
+            b = b * cn - a * sn;
+            a = an;
+            if (surv == 0) {
+                land();
+                live = false;
+            }
+        } else {
+            // skipped particle: the reference's Cartesian round trip
+            double sinFi, cosFi;
+            sincos(fi, &sinFi, &cosFi);
+            const double x = r * cosFi, y = r * sinFi;
+            const double vx = a * cosFi - r * b * sinFi;
+            const double vy = a * sinFi + r * b * cosFi;
+            const double rn = sqrt(x * x + y * y);
+            a = vx * cosFi + vy * sinFi;
+            const double vfi = -vx * sinFi + vy * cosFi;
+            b = rn > 1e-12 ? vfi / rn : 0.0;
+            r = rn;
+            ir = 1.0 / rn;
+        }
+        rfph += __ldg(drf + s);
+        if constexpr (XING) {
+            if (surv0 == 1) {
+                const double post[7] = {r, live ? a * ig : a, z, live ? c * ig : c, fi,
+                                        live ? (r > 1e-12 ? b * ig * ir : 0.0) : b, rfph};
+                if (!SC) { esr = S.esc_r[i]; esz = S.esc_z[i]; esf = S.esc_fi[i]; }
+                xing_check(p.xing, i, p.step0 + s, pre, post, surv, inj, esr, esz, esf, p.dt);
+            }
+        }
+    }
+    if (live) land();
+    S.r[i] = r; S.vr[i] = a; S.z[i] = z; S.vz[i] = c; S.fi[i] = fi; S.f5[i] = b;
+    S.rf[i] = rfph;
+    if (SC) { S.esc_r[i] = esr; S.esc_z[i] = esz; S.esc_fi[i] = esf; }
+    S.inj[i] = (uint8_t)inj;
+    S.surv[i] = (uint8_t)surv;
+    status_add(p.status, lost, !(isfinite(r) && isfinite(fi) && isfinite(z)), oob);
+}
+
+// The FP32C step: the float32 field under the reference's velocity form of the
+// push, as all its stored results were made.  NREG: the register cap.  80 is
+// the default launch shape; the compensated
 // float32 pusher without space charge is also built with 72, 64 and 56
 // (more resident warps, more spills) for the launch-shape autotuner.  The
 // cap changes register allocation only, not the arithmetic.
-template <int MAXO, bool SC, bool XING, bool F32, int NREG = 80, bool HARM = false>
-__global__ void __maxnreg__(NREG) boris_f64_kernel(const __grid_constant__ PushK p)
+template <int MAXO, bool SC, bool XING, int NREG = 80, bool HARM = false>
+__global__ void __maxnreg__(NREG) boris_f32c_kernel(const __grid_constant__ PushK p)
 {
     const int64_t t_ = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t_ >= p.n) return;
@@ -671,7 +973,7 @@ __global__ void __maxnreg__(NREG) boris_f64_kernel(const __grid_constant__ PushK
     for (int s = 0; s < p.nsteps; ++s) {
         const int64_t gs = p.step0 + s;
         if (injs == gs) { inj = 1; surv = 1; }
-        if (SC) ex.apply(gs, p.sc_step, esr, esz, esf);
+        if (SC) ex.apply(sc_phase(p, gs), p.inv_sc, esr, esz, esf);
         const double drf = __ldg(p.drf + gs);
         double pre[7];
         const int surv0 = surv;
@@ -686,19 +988,7 @@ __global__ void __maxnreg__(NREG) boris_f64_kernel(const __grid_constant__ PushK
             // periodic field (0 and the period)
             const double fim = fi - f.period * floor(fi * f.inv_period);
             double Bz, Br, Bfi;
-            if constexpr (F32) {
-                field_mixed<MAXO>(f, r, ir, fim, z, Bz, Br, Bfi, oob);
-            } else {
-                // the table lookup first: its loads are in flight while the
-                // analytic part computes (measured 3.53 vs 3.64 ms per
-                // 1e5-particle turn; 3.30 ms with the zero-spiral skip)
-                double hz = 0.0, hf = 0.0, hr = 0.0;
-                if constexpr (MAXO >= 1) high_order_b64<MAXO>(f, r, fim, z, hz, hf, hr, oob);
-                analytic_b64(f, r, ir, fim, z, Bz, Br, Bfi);
-                Bz += hz;
-                Bfi += hf;
-                Br += hr;
-            }
+            field_mixed<MAXO>(f, r, ir, fim, z, Bz, Br, Bfi, oob);
             if constexpr (HARM) Bz += harmonics_bz(f.harm, f.n_harm, r, fi);
             double Er, Ez, Efi;
             rf_field64(p.rf, acc, r, fi, z, rfph, Er, Ez, Efi);
@@ -1021,8 +1311,7 @@ __device__ __forceinline__ void rk4_rhs64(const PushK &p, const Y7 &y, double ra
     if constexpr (F32) {
         field_mixed<MAXO>(f, y.r, 1.0 / y.r, fim, y.z, Bz, Br, Bfi, oob);
     } else {
-        analytic_b64(f, y.r, 1.0 / y.r, fim, y.z, Bz, Br, Bfi);
-        if constexpr (MAXO >= 1) high_order_b64<MAXO>(f, y.r, fim, y.z, Bz, Bfi, Br, oob);
+        field64<MAXO>(f, y.r, 1.0 / y.r, fim, y.z, Bz, Br, Bfi, oob);
     }
     if constexpr (HARM) Bz += harmonics_bz(f.harm, f.n_harm, y.r, y.fi);
     double Er, Ez, Efi;
@@ -1071,7 +1360,7 @@ __global__ void __maxnreg__(80) rk4_f64_kernel(const __grid_constant__ PushK p)
     for (int s = 0; s < p.nsteps; ++s) {
         const int64_t gs = p.step0 + s;
         if (injs == gs) { inj = 1; surv = 1; }
-        if (SC) ex.apply(gs, p.sc_step, esr, esz, esf);
+        if (SC) ex.apply(sc_phase(p, gs), p.inv_sc, esr, esz, esf);
         const double *rate = p.drf + 4 * gs;
         const double *acc = p.acc + 4 * gs;
         const double k1rf = h * __ldg(rate + 0), k2rf = h * __ldg(rate + 1);
@@ -1143,7 +1432,8 @@ __device__ __forceinline__ void seo_rhs(const FieldK &f, double t, const double 
     const double fim = fmod(fi, f.period);
     const double r = x[0], pr = x[1], z = x[2], pz = x[3];
     double Bz, Br, Bfi;
-    analytic_b64(f, r, 1.0 / r, fim, z, Bz, Br, Bfi);
+    int clamped = 0;
+    field64<0>(f, r, 1.0 / r, fim, z, Bz, Br, Bfi, clamped);
     const double pfi = sqrt(1.0 - pr * pr - pz * pz);
     const double qP = q / P;
     d[0] = r * pr / pfi;
@@ -1172,7 +1462,8 @@ __global__ void __launch_bounds__(64) theta_track_kernel(const __grid_constant__
             row[2] = x[2];
             row[3] = x[3];
             const double fim = fmod(fmod(ts, 2.0 * PI), f.period);
-            analytic_b64(f, x[0], 1.0 / x[0], fim, x[2], row[4], row[5], row[6]);
+            int clamped = 0;
+            field64<0>(f, x[0], 1.0 / x[0], fim, x[2], row[4], row[5], row[6], clamped);
         }
     };
     if (tr) record(0, 0.0);
@@ -1217,7 +1508,8 @@ __global__ void pack_nodes_kernel(const double *__restrict__ bz, const double *_
             const double *src = comp == 0 ? bz : (comp == 1 ? bfi : br);
             val = src[(int64_t)n * plane + node];
         }
-        n64[node * npad + v] = val;
+        const int a = v & ~3, w = map_plane_width(max_order, a);
+        if (v - a < w) n64[a * plane + node * w + (v - a)] = val;
         n32[node * npad + v] = (float)val;
     }
 }
@@ -1231,26 +1523,52 @@ cudaError_t launch_pack_nodes(const ffa_field_desc &d, int npad, double *n64, fl
     return cudaGetLastError();
 }
 
-// Field-error harmonics select their own kernel variants (HARM), so that
-// the harmonic sum costs the common case nothing.
-template <int MAXO, bool SC, bool F32>
-static void boris_default(const PushK &p, cudaStream_t s, int tb)
+// Register cap of a float64 Boris launch of n particles.  More registers
+// keep more of a step's loads and chains in flight per warp, fewer hold more
+// warps; 80, 128 and 255 leave 24, 16 and 8 warps per SM.  What decides is how
+// many waves the warps make (us per 180 steps, z-Taylor order 2, RF, 148 SMs):
+//   particles     10000  56800  75000  100000  113600  150000  300000  1000000
+//   80 registers    252    276    303     375     376     610     980     2971
+//   128 registers   199    221    254     418     431     480     929     2996
+//   255 registers   198    219    405     417     425     605    1162     3608
+// so 128 up to 16 warps per SM, 80 while that is one wave, and 128 again
+// beyond.  From order 3 a step's node loads alone need more than 128 (order 4,
+// 10000 particles, 720 steps: 935 us with 128, 791 us with 255).  With space
+// charge the endpoints' registers make 80 spill (60 steps, 1e6 particles: 1898
+// us, 1627 us with 128; 100000: 227 and 224).
+static int boris_cap(const PushK &p, bool sc, int max_order)
 {
-    const unsigned g = (unsigned)((p.n + tb - 1) / tb);
-    const bool x = xing_on(p);
-    if (p.f.n_harm > 0) {
-        if (x) boris_f64_kernel<MAXO, SC, true, F32, 80, true><<<g, tb, 0, s>>>(p);
-        else boris_f64_kernel<MAXO, SC, false, F32, 80, true><<<g, tb, 0, s>>>(p);
-    } else {
-        if (x) boris_f64_kernel<MAXO, SC, true, F32><<<g, tb, 0, s>>>(p);
-        else boris_f64_kernel<MAXO, SC, false, F32><<<g, tb, 0, s>>>(p);
-    }
+    if (sc) return 128;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t warps = (p.n + 31) / 32;
+    if (max_order >= 3 && warps <= (int64_t)8 * sms) return 255;
+    if (warps <= (int64_t)16 * sms) return 128;
+    return warps <= (int64_t)24 * sms ? 80 : 128;
 }
 
+template <int MAXO, bool SC, int NREG, bool HARM>
+static void boris_shaped(const PushK &p, cudaStream_t s, int tb)
+{
+    const unsigned g = (unsigned)((p.n + tb - 1) / tb);
+    if (xing_on(p)) boris_f64_kernel<MAXO, SC, true, NREG, HARM><<<g, tb, 0, s>>>(p);
+    else boris_f64_kernel<MAXO, SC, false, NREG, HARM><<<g, tb, 0, s>>>(p);
+}
+
+// Field-error harmonics select their own kernel variants (HARM), so that
+// the harmonic sum costs the common case nothing.
 template <int MAXO, bool SC>
 static void boris_launch(const PushK &p, cudaStream_t s, int tb, int)
 {
-    boris_default<MAXO, SC, false>(p, s, tb);
+    if (p.f.n_harm > 0) return boris_shaped<MAXO, SC, 128, true>(p, s, tb);
+    const int cap = boris_cap(p, SC, MAXO);
+    if constexpr (!SC) {
+        if (cap == 80) return boris_shaped<MAXO, SC, 80, false>(p, s, tb);
+        if constexpr (MAXO >= 3) {
+            if (cap == 255) return boris_shaped<MAXO, SC, 255, false>(p, s, tb);
+        }
+    }
+    boris_shaped<MAXO, SC, 128, false>(p, s, tb);
 }
 
 template <int MAXO, bool SC, bool F32>
@@ -1302,7 +1620,7 @@ cudaError_t launch_rk4_f64(const PushK &p, cudaStream_t s, bool f32)
 template <int MAXO, bool XING, int NREG>
 static void boris32_shaped(const PushK &p, cudaStream_t s, int tb)
 {
-    boris_f64_kernel<MAXO, false, XING, true, NREG><<<(unsigned)((p.n + tb - 1) / tb), tb, 0, s>>>(p);
+    boris_f32c_kernel<MAXO, false, XING, NREG><<<(unsigned)((p.n + tb - 1) / tb), tb, 0, s>>>(p);
 }
 
 template <int MAXO, bool SC>
@@ -1319,7 +1637,15 @@ static void boris32_launch(const PushK &p, cudaStream_t s, int tb, int nreg_sel)
             return;
         }
     }
-    boris_default<MAXO, SC, true>(p, s, tb);
+    const unsigned g = (unsigned)((p.n + tb - 1) / tb);
+    const bool x = xing_on(p);
+    if (p.f.n_harm > 0) {
+        if (x) boris_f32c_kernel<MAXO, SC, true, 80, true><<<g, tb, 0, s>>>(p);
+        else boris_f32c_kernel<MAXO, SC, false, 80, true><<<g, tb, 0, s>>>(p);
+    } else {
+        if (x) boris_f32c_kernel<MAXO, SC, true><<<g, tb, 0, s>>>(p);
+        else boris_f32c_kernel<MAXO, SC, false><<<g, tb, 0, s>>>(p);
+    }
 }
 
 cudaError_t launch_boris_f32c(const PushK &p, cudaStream_t s, int tb, int nreg_sel)
@@ -1354,12 +1680,12 @@ static const void *push_kernel_fn(bool rk4, bool f32, int nreg_sel)
 {
     if (rk4) return f32 ? (const void *)rk4_f64_kernel<MAXO, false, X, false, true>
                         : (const void *)rk4_f64_kernel<MAXO, false, X>;
-    if (!f32) return (const void *)boris_f64_kernel<MAXO, false, X, false>;
+    if (!f32) return (const void *)boris_f64_kernel<MAXO, false, X, 80>;
     switch (nreg_sel) {
-    case 0: return (const void *)boris_f64_kernel<MAXO, false, X, true, 80>;
-    case 1: return (const void *)boris_f64_kernel<MAXO, false, X, true, 72>;
-    case 2: return (const void *)boris_f64_kernel<MAXO, false, X, true, 64>;
-    default: return (const void *)boris_f64_kernel<MAXO, false, X, true, 56>;
+    case 0: return (const void *)boris_f32c_kernel<MAXO, false, X, 80>;
+    case 1: return (const void *)boris_f32c_kernel<MAXO, false, X, 72>;
+    case 2: return (const void *)boris_f32c_kernel<MAXO, false, X, 64>;
+    default: return (const void *)boris_f32c_kernel<MAXO, false, X, 56>;
     }
 }
 
