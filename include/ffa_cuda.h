@@ -278,7 +278,7 @@ int ffa_push(const ffa_fieldmap *fm, const ffa_rf_desc *rf, const ffa_aperture *
  * ffa_push / ffa_push_crossing (crossing != 0) would launch for `flags` and
  * a field map of `max_order`, without space charge (the runtime's occupancy
  * calculator; needs a device; float64 Boris: the kernel of a bunch that fills
- * the device once -- others run it with more registers).  For the launch-shape autotuner's report.
+ * the device once, RK4: that of a large one -- others run with more registers).  For the launch-shape autotuner's report.
  * No counterpart in the reference, whose Numba kernels have no launch shape. */
 int ffa_push_occupancy(int32_t flags, int32_t max_order, int32_t crossing, int32_t *blocks_per_sm,
                        int32_t *threads_per_block);

@@ -1296,23 +1296,133 @@ struct Y7 {
     double r, vr, z, vz, fi, E, rf;
 };
 
+// The FP64 stage: RK4_equations_of_motion_njit for one live particle.  What
+// depends on the energy alone (v^2, q c^2 / E) is carried and formed anew only
+// where the stage's energy differs from the last one, i.e. in an electric
+// field; one reciprocal (1 / r) and one inverse square root are left of the
+// seven divisions and square roots of the reference's form.  The stages are
+// one loop, so the right-hand side is in the code once (four inlined copies
+// miss the instruction cache); stage k is evaluated at y + a h d(k-1) with
+// a = 1/2, 1/2, 1 and the derivatives are summed as d1 + 2 d2 + 2 d3 + d4.
+// Bound as the Boris step (boris_f64_kernel): the node loads' latency and the
+// chain behind them, four times a step.  1e5 particles, 720 steps, order 2, RF:
+// 9.2 -> 5.6 ms (11.3 ms before field64).
+template <int MAXO, bool SC, bool XING, int NREG, bool HARM = false>
+__global__ void __maxnreg__(NREG) rk4_f64_kernel(const __grid_constant__ PushK p)
+{
+    const int64_t t_ = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t_ >= p.n) return;
+    const int64_t i = p.st.order ? (int64_t)__ldg(p.st.order + t_) : t_;   // the particle this thread advances
+    const FieldK &f = p.f;
+    const ffa_state_soa &S = p.st;
+    double r = S.r[i], vr = S.vr[i], z = S.z[i], vz = S.vz[i], fi = S.fi[i], E = S.f5[i], rf = S.rf[i];
+    double esr = S.esc_r[i], esz = S.esc_z[i], esf = S.esc_fi[i];
+    const bool esc = SC || esr != 0.0 || esz != 0.0 || esf != 0.0;   // also for NaN
+    int inj = S.inj[i], surv = S.surv[i];
+    const int32_t injs = S.inj_step ? S.inj_step[i] : -1;
+    SCExtrap ex;
+    if (SC) ex.load(S, i);
+    const double h = p.dt, h6 = p.dt * (1.0 / 6.0), c2 = p.cs.c * p.cs.c, q = p.cs.q;
+    double Ev = 0.0, v2 = 0.0, qc2E = 0.0;       // the energy these two belong to
+    int oob = 0;
+    for (int s = 0; s < p.nsteps; ++s) {
+        const int64_t gs = p.step0 + s;
+        if (injs == gs) { inj = 1; surv = 1; }
+        if (SC) ex.apply(sc_phase(p, gs), p.inv_sc, esr, esz, esf);
+        const double *rate = p.drf + 4 * gs;
+        double pre[7];
+        if constexpr (XING) {
+            pre[0] = r; pre[1] = vr; pre[2] = z; pre[3] = vz; pre[4] = fi; pre[5] = E; pre[6] = rf;
+        }
+        const double drf = h6 * (__ldg(rate) + 2 * __ldg(rate + 1) + 2 * __ldg(rate + 2) + __ldg(rate + 3));
+        if (inj == 1 && surv == 1) {
+            double sr = 0.0, svr = 0.0, sz = 0.0, svz = 0.0, sfi = 0.0, sE = 0.0;
+            double yr = r, yvr = vr, yz = z, yvz = vz, yfi = fi, yE = E, yrf = rf;
+#pragma unroll 1
+            for (int k = 0; k < 4; ++k) {
+                const double fim = yfi - f.period * floor(yfi * f.inv_period);
+                const double ir = rcp64(yr);
+                double Bz, Br, Bfi;
+                field64<MAXO>(f, yr, ir, fim, yz, Bz, Br, Bfi, oob);
+                if constexpr (HARM) Bz += harmonics_bz(f.harm, f.n_harm, yr, yfi);
+                if (yE != Ev) {
+                    const double iE = 1.0 / yE, ig = p.cs.E0 * iE;
+                    Ev = yE;
+                    v2 = (1.0 - ig * ig) * c2;
+                    qc2E = q * c2 * iE;
+                }
+                const double vp2 = v2 - yvr * yvr - yvz * yvz;
+                const double vp = vp2 * rsqrt64(vp2);
+                const double w = vp * ir;                        // d(fi)/dt
+                double dvr = vp * w + qc2E * (yvz * Bfi - vp * Bz);
+                double dvz = qc2E * (vp * Br - yvr * Bfi);
+                double dE = 0.0;
+                double3 e = make_double3(0.0, 0.0, 0.0);
+                const bool hit = rf_hit64(p.rf, p.acc + 4 * gs + k, yr, yfi, yz, yrf, e);
+                if (esc || hit) {
+                    if (esc) {
+                        if (!SC) { esr = S.esc_r[i]; esz = S.esc_z[i]; esf = S.esc_fi[i]; }   // not held over the loop
+                        e.x += esr;
+                        e.y += esz;
+                        e.z += esf;
+                    }
+                    const double P = yvr * e.x + vp * e.z + yvz * e.y, c = q / yE * P;
+                    dvr += qc2E * e.x - yvr * c;
+                    dvz += qc2E * e.y - yvz * c;
+                    dE = q * P;
+                }
+                const double wk = (k == 1 || k == 2) ? 2.0 : 1.0, ah = k == 2 ? h : 0.5 * h;
+                sr = fma(wk, yvr, sr);
+                svr = fma(wk, dvr, svr);
+                sz = fma(wk, yvz, sz);
+                svz = fma(wk, dvz, svz);
+                sfi = fma(wk, w, sfi);
+                sE = fma(wk, dE, sE);
+                yr = fma(ah, yvr, r);
+                yz = fma(ah, yvz, z);
+                yvr = fma(ah, dvr, vr);
+                yvz = fma(ah, dvz, vz);
+                yfi = fma(ah, w, fi);
+                yE = fma(ah, dE, E);
+                yrf = fma(ah, __ldg(rate + k), rf);
+            }
+            r = fma(h6, sr, r);
+            vr = fma(h6, svr, vr);
+            z = fma(h6, sz, z);
+            vz = fma(h6, svz, vz);
+            fi = fma(h6, sfi, fi);
+            E = fma(h6, sE, E);
+        }
+        rf += drf;
+        if constexpr (XING) {
+            if (surv == 1) {
+                const double post[7] = {r, vr, z, vz, fi, E, rf};
+                if (!SC) { esr = S.esc_r[i]; esz = S.esc_z[i]; esf = S.esc_fi[i]; }
+                xing_check(p.xing, i, gs, pre, post, surv, inj, esr, esz, esf, p.dt);
+            }
+        }
+    }
+    S.r[i] = r; S.vr[i] = vr; S.z[i] = z; S.vz[i] = vz; S.fi[i] = fi; S.f5[i] = E;
+    S.rf[i] = rf;
+    if (SC) { S.esc_r[i] = esr; S.esc_z[i] = esz; S.esc_fi[i] = esf; }
+    S.inj[i] = (uint8_t)inj;
+    S.surv[i] = (uint8_t)surv;
+    status_add(p.status, 0, !(isfinite(r) && isfinite(fi) && isfinite(z)), oob);
+}
+
 // RK4_equations_of_motion_njit for one live particle at stage state y.
-// F32: the field of the FP32C Boris pusher (field_mixed: float32 flutter
+// FP32C: the field of the FP32C Boris pusher (field_mixed: float32 flutter
 // exponentials and map lookup, float64 products with r and z); the
 // equations of motion and the RK4 stages stay float64.
-template <int MAXO, bool HARM, bool F32>
-__device__ __forceinline__ void rk4_rhs64(const PushK &p, const Y7 &y, double rate, double acc,
+template <int MAXO, bool HARM>
+__device__ __forceinline__ void rk4_rhs_f32c(const PushK &p, const Y7 &y, double rate, double acc,
                                           double esr, double esz, double esf, Y7 &d, int &oob)
 {
     const FieldK &f = p.f;
     const double q = p.cs.q, c = p.cs.c, E0 = p.cs.E0;
     const double fim = y.fi - f.period * floor(y.fi / f.period);
     double Bz, Br, Bfi;
-    if constexpr (F32) {
-        field_mixed<MAXO>(f, y.r, 1.0 / y.r, fim, y.z, Bz, Br, Bfi, oob);
-    } else {
-        field64<MAXO>(f, y.r, 1.0 / y.r, fim, y.z, Bz, Br, Bfi, oob);
-    }
+    field_mixed<MAXO>(f, y.r, 1.0 / y.r, fim, y.z, Bz, Br, Bfi, oob);
     if constexpr (HARM) Bz += harmonics_bz(f.harm, f.n_harm, y.r, y.fi);
     double Er, Ez, Efi;
     rf_field64(p.rf, acc, y.r, y.fi, y.z, y.rf, Er, Ez, Efi);
@@ -1335,15 +1445,15 @@ __device__ __forceinline__ void rk4_rhs64(const PushK &p, const Y7 &y, double ra
     d.rf = rate;
 }
 
-// One-warp blocks (RK4_TB), at most 80 registers (24 warps per SM, spills
+// FP32C: one-warp blocks (RK4_TB), at most 80 registers (24 warps per SM, spills
 // to L1): the 3125 warps of a 1e5-particle bunch are resident in one wave.
 // Uncapped the kernel takes 130 registers, 12 warps per SM, 1.76 waves
 // (measured on c1: 14.8 ms per 720-step turn uncapped; at 80 registers
 // 12.4 ms in 128-thread blocks, 12.3 ms in 32-thread blocks; 11.3 ms with
 // the stages as one loop, whose loop body the instruction cache holds).
 
-template <int MAXO, bool SC, bool XING, bool HARM = false, bool F32 = false>
-__global__ void __maxnreg__(80) rk4_f64_kernel(const __grid_constant__ PushK p)
+template <int MAXO, bool SC, bool XING, bool HARM = false>
+__global__ void __maxnreg__(80) rk4_f32c_kernel(const __grid_constant__ PushK p)
 {
     const int64_t t_ = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t_ >= p.n) return;
@@ -1385,7 +1495,7 @@ __global__ void __maxnreg__(80) rk4_f64_kernel(const __grid_constant__ PushK p)
         Y7 d, K, S, ys = y;
 #pragma unroll 1
         for (int k = 0; k < 4; ++k) {
-            rk4_rhs64<MAXO, HARM, F32>(p, ys, __ldg(rate + k), __ldg(acc + k), esr, esz, esf, d, oob);
+            rk4_rhs_f32c<MAXO, HARM>(p, ys, __ldg(rate + k), __ldg(acc + k), esr, esz, esf, d, oob);
             K = {h * d.r, h * d.vr, h * d.z, h * d.vz, h * d.fi, h * d.E, h * d.rf};
             if (k == 0) {
                 S = K;
@@ -1571,26 +1681,59 @@ static void boris_launch(const PushK &p, cudaStream_t s, int tb, int)
     boris_shaped<MAXO, SC, 128, false>(p, s, tb);
 }
 
-template <int MAXO, bool SC, bool F32>
-static void rk4_launch_p(const PushK &p, cudaStream_t s)
+// Register cap of a float64 RK4 launch of n particles: 255, 168 or 128 leave 8,
+// 12 or 16 warps per SM, and a wave of them takes about 0.69, 0.83 and 1 of
+// the time (with space charge 0.60, 0.72 and 1); the cap with the least total
+// over its waves.  Measured (us per 180 steps, z-Taylor order 2, RF, 148 SMs):
+//   particles     10000  37800  56800  75000  100000  150000  200000  1000000
+//   128 registers   605    652    741    846    1448    1619    2278    10379
+//   168 registers   570    624    704   1269    1308    1912    2516    11481
+//   255 registers   528    583   1113   1156    1657    2236    3220    14586
+// (80 registers spill the stages: 806 and 1718 us at 10000 and 100000)
+static int rk4_cap(const PushK &p, bool sc)
 {
-    const int tb = RK4_TB;
-    const unsigned g = (unsigned)((p.n + tb - 1) / tb);
-    const bool x = xing_on(p);
-    if (p.f.n_harm > 0) {
-        if (x) rk4_f64_kernel<MAXO, SC, true, true, F32><<<g, tb, 0, s>>>(p);
-        else rk4_f64_kernel<MAXO, SC, false, true, F32><<<g, tb, 0, s>>>(p);
-    } else {
-        if (x) rk4_f64_kernel<MAXO, SC, true, false, F32><<<g, tb, 0, s>>>(p);
-        else rk4_f64_kernel<MAXO, SC, false, false, F32><<<g, tb, 0, s>>>(p);
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t warps = (p.n + 31) / 32;
+    const int cap[3] = {128, 168, 255}, per_sm[3] = {16, 12, 8}, cost[2][3] = {{100, 83, 69}, {100, 72, 60}};
+    int best = 0;
+    int64_t least = INT64_MAX;
+    for (int v = 0; v < 3; ++v) {
+        const int64_t room = (int64_t)per_sm[v] * sms, t = (warps + room - 1) / room * cost[sc][v];
+        if (t < least) { least = t; best = v; }
     }
+    return cap[best];
+}
+
+template <int MAXO, bool SC, int NREG, bool HARM>
+static void rk4_shaped(const PushK &p, cudaStream_t s)
+{
+    const unsigned g = (unsigned)((p.n + RK4_TB - 1) / RK4_TB);
+    if (xing_on(p)) rk4_f64_kernel<MAXO, SC, true, NREG, HARM><<<g, RK4_TB, 0, s>>>(p);
+    else rk4_f64_kernel<MAXO, SC, false, NREG, HARM><<<g, RK4_TB, 0, s>>>(p);
 }
 
 template <int MAXO, bool SC>
 static void rk4_launch(const PushK &p, cudaStream_t s, bool f32)
 {
-    if (f32) rk4_launch_p<MAXO, SC, true>(p, s);
-    else rk4_launch_p<MAXO, SC, false>(p, s);
+    if (f32) {
+        const unsigned g = (unsigned)((p.n + RK4_TB - 1) / RK4_TB);
+        const bool x = xing_on(p);
+        if (p.f.n_harm > 0) {
+            if (x) rk4_f32c_kernel<MAXO, SC, true, true><<<g, RK4_TB, 0, s>>>(p);
+            else rk4_f32c_kernel<MAXO, SC, false, true><<<g, RK4_TB, 0, s>>>(p);
+        } else {
+            if (x) rk4_f32c_kernel<MAXO, SC, true><<<g, RK4_TB, 0, s>>>(p);
+            else rk4_f32c_kernel<MAXO, SC, false><<<g, RK4_TB, 0, s>>>(p);
+        }
+        return;
+    }
+    if (p.f.n_harm > 0) return rk4_shaped<MAXO, SC, 128, true>(p, s);
+    switch (rk4_cap(p, SC)) {
+    case 255: return rk4_shaped<MAXO, SC, 255, false>(p, s);
+    case 168: return rk4_shaped<MAXO, SC, 168, false>(p, s);
+    default: return rk4_shaped<MAXO, SC, 128, false>(p, s);
+    }
 }
 
 #define FFA_DISPATCH(FN, p, ...)                                                       \
@@ -1678,8 +1821,7 @@ cudaError_t launch_boris_f32(const PushK &p, cudaStream_t s, int tb)
 template <int MAXO, bool X>
 static const void *push_kernel_fn(bool rk4, bool f32, int nreg_sel)
 {
-    if (rk4) return f32 ? (const void *)rk4_f64_kernel<MAXO, false, X, false, true>
-                        : (const void *)rk4_f64_kernel<MAXO, false, X>;
+    if (rk4) return f32 ? (const void *)rk4_f32c_kernel<MAXO, false, X> : (const void *)rk4_f64_kernel<MAXO, false, X, 128>;
     if (!f32) return (const void *)boris_f64_kernel<MAXO, false, X, 80>;
     switch (nreg_sel) {
     case 0: return (const void *)boris_f32c_kernel<MAXO, false, X, 80>;
