@@ -121,12 +121,69 @@ __device__ __noinline__ double power_direct(const FieldK &f, double r) { return 
 // latency and issue.  Measured (720 steps, z-Taylor order 2, RF): 1e5
 // particles Boris 2.47 -> 2.07 ms, RK4 11.3 -> 9.6 ms; 1e4 particles, order 4:
 // 1.87 -> 1.74 ms; 1280 azimuth-domain tracks of 523 steps: 2.46 -> 1.59 ms.
+// One flutter cell and the position in it
+struct FlutterCell {
+    double c[8], x;
+};
+
+// Cell j covers [j, j + 1) cells of azimuth; one guard cell on each side
+// takes a reduction that rounded just outside the sector.
+__device__ __forceinline__ FlutterCell flutter_fetch(const FieldK &f, double fs)
+{
+    FlutterCell t;
+    const double q = fma(fs, f.fl_scale, -0.5), qi = q + INT_MAGIC;
+    const int j = min(max(__double2loint(qi) + 1, 0), f.fl_n - 1);
+    t.x = q - (qi - INT_MAGIC);
+    ldg_v4(f.fl_tab + 8 * j, t.c);
+    ldg_v4(f.fl_tab + 8 * j + 4, t.c + 4);
+    return t;
+}
+
+__device__ __forceinline__ void flutter_eval(const FieldK &f, const FlutterCell &t, double &F, double &Fp)
+{
+    F = t.c[7];
+    Fp = 0.0;
+#pragma unroll
+    for (int a = 6; a >= 0; --a) {
+        Fp = (a == 6) ? F : fma(Fp, t.x, F);
+        F = fma(F, t.x, t.c[a]);
+    }
+    Fp *= f.fl_scale;
+}
+
+// One power entry (B0 r_j^(k-1), 1 / r_j), r - r_j, and whether r is inside
+// the table
+struct PowerEntry {
+    double2 e;
+    double d;
+    bool in;
+};
+
+__device__ __forceinline__ PowerEntry power_fetch(const FieldK &f, double r)
+{
+    PowerEntry t;
+    const double pi = fma(r, f.pw_scale, INT_MAGIC);
+    const int k = __double2loint(pi) - f.pw_j0;
+    t.in = __double2hiint(pi) == INT_HI && (unsigned)k < (unsigned)f.pw_n;
+    t.d = fma(INT_MAGIC - pi, f.pw_h, r);
+    t.e = __ldg(f.pw_tab + (t.in ? k : 0));
+    return t;
+}
+
+// B0 r^(k-1)
+__device__ __forceinline__ double power_eval(const FieldK &f, const PowerEntry &t, double r)
+{
+    const double u = t.d * t.e.y;
+    const double P = fma(u, fma(u, fma(u, f.pw_c[3], f.pw_c[2]), f.pw_c[1]), f.pw_c[0]);
+    double G = fma(t.e.x * u, P, t.e.x);
+    if (!t.in) G = power_direct(f, r);
+    return G;
+}
+
 struct Tables {
-    double c[8], x;      // flutter cell and the position in it
-    double2 e;           // power entry (B0 r_j^(k-1), 1 / r_j)
-    double d;            // r - r_j
+    FlutterCell fl;
+    PowerEntry pw;
     double fs, spiral_p;
-    bool pw;             // r is inside the power table
 };
 
 // The table entries of a point, loaded unconditionally (a map without a table
@@ -149,18 +206,8 @@ __device__ __forceinline__ Tables tables_fetch(const FieldK &f, double ri, doubl
         t.fs = fim - spiral;
         t.fs -= f.period * floor(t.fs * f.inv_period);
     }
-    // cell j covers [j, j + 1) cells of azimuth; one guard cell on each side
-    // takes a reduction that rounded just outside the sector
-    const double q = fma(t.fs, f.fl_scale, -0.5), qi = q + INT_MAGIC;
-    const int j = min(max(__double2loint(qi) + 1, 0), f.fl_n - 1);
-    t.x = q - (qi - INT_MAGIC);
-    ldg_v4(f.fl_tab + 8 * j, t.c);
-    ldg_v4(f.fl_tab + 8 * j + 4, t.c + 4);
-    const double pi = fma(ri, f.pw_scale, INT_MAGIC);
-    const int k = __double2loint(pi) - f.pw_j0;
-    t.pw = __double2hiint(pi) == INT_HI && (unsigned)k < (unsigned)f.pw_n;
-    t.d = fma(INT_MAGIC - pi, f.pw_h, ri);
-    t.e = __ldg(f.pw_tab + (t.pw ? k : 0));
+    t.fl = flutter_fetch(f, t.fs);
+    t.pw = power_fetch(f, ri);
     return t;
 }
 
@@ -168,18 +215,8 @@ __device__ __forceinline__ Tables tables_fetch(const FieldK &f, double ri, doubl
 __device__ __forceinline__ void tables_eval(const FieldK &f, const Tables &t, double ri, double &F, double &Fp,
                                             double &G, double &kG)
 {
-    F = t.c[7];
-    Fp = 0.0;
-#pragma unroll
-    for (int a = 6; a >= 0; --a) {
-        Fp = (a == 6) ? F : fma(Fp, t.x, F);
-        F = fma(F, t.x, t.c[a]);
-    }
-    Fp *= f.fl_scale;
-    const double u = t.d * t.e.y;
-    const double P = fma(u, fma(u, fma(u, f.pw_c[3], f.pw_c[2]), f.pw_c[1]), f.pw_c[0]);
-    G = fma(t.e.x * u, P, t.e.x);
-    if (!t.pw) G = power_direct(f, ri);
+    flutter_eval(f, t.fl, F, Fp);
+    G = power_eval(f, t.pw, ri);
     kG = f.k * G;
     if (f.unusual) {                     // no flutter table, or a field index of 0
         if (f.fl_direct) {
@@ -1532,33 +1569,51 @@ __global__ void __maxnreg__(80) rk4_f32c_kernel(const __grid_constant__ PushK p)
 
 // ------------------------------------------------- closed-orbit tracks
 
-// d/dtheta of (r, pr, z, pz) at fixed momentum P (FunctionForSEO,
-// src/FFAG_track.py:1698-1740), same operation order.
-__device__ __forceinline__ void seo_rhs(const FieldK &f, double t, const double x[4], double P, double q,
-                                        double d[4])
+// An azimuth t >= 0 reduced mod 2 pi and then mod the sector, as the
+// reference's fmod pair does; a multiple that rounding puts off by one leaves
+// a value just outside the sector, where the field is the same.  Every
+// track of a launch has the same t, so this is off their chains.
+__device__ __forceinline__ double sector_azimuth(const FieldK &f, double t)
 {
     const double tw = 2.0 * PI;
-    const double fi = fmod(t, tw);
-    const double fim = fmod(fi, f.period);
-    const double r = x[0], pr = x[1], z = x[2], pz = x[3];
-    double Bz, Br, Bfi;
-    int clamped = 0;
-    field64<0>(f, r, 1.0 / r, fim, z, Bz, Br, Bfi, clamped);
-    const double pfi = sqrt(1.0 - pr * pr - pz * pz);
-    const double qP = q / P;
-    d[0] = r * pr / pfi;
-    d[1] = pfi - qP * (r * Bz - r * pz / pfi * Bfi);
-    d[2] = r * pz / pfi;
-    d[3] = qP * (r * Br - r * pr / pfi * Bfi);
+    const double fi = fma(-tw, floor(t * (0.5 / PI)), t);
+    return fma(-f.period, floor(fi * f.inv_period), fi);
 }
 
-__global__ void __launch_bounds__(64) theta_track_kernel(const __grid_constant__ FieldK f,
+// d/dtheta of (r, pr, z, pz) at fixed momentum P (FunctionForSEO,
+// src/FFAG_track.py:1698-1740), qP = q / P, from the flutter F, F', G = B0
+// r^(k-1) and kG = k G.  The field enters only times r, which cancels the 1 / r
+// of Bfi.
+__device__ __forceinline__ void seo_rhs(const double x[4], double qP, double F, double Fp, double G, double kG,
+                                        double spiral_p, double d[4])
+{
+    const double r = x[0], pr = x[1], z = x[2], pz = x[3];
+    const double pf2 = 1.0 - pr * pr - pz * pz, ipf = rsqrt64(pf2);
+    const double Gr = G * r, rBz = Gr * r * F, rBfi = Gr * Fp * z;
+    const double rBr = r * fma(kG, F, -Gr * Fp * spiral_p) * z;
+    const double ur = pr * ipf, uz = pz * ipf;
+    d[0] = r * ur;
+    d[1] = fma(pf2, ipf, qP * (uz * rBfi - rBz));
+    d[2] = r * uz;
+    d[3] = qP * (rBr - ur * rBfi);
+}
+
+// One thread per track; a scan has a few thousand of them, so the launch is
+// one step's chain long whatever the chip could hold: power-table load
+// (about 40 cycles from L1), field, inverse square root, stage update.  One
+// warp per block, so that the warps spread over the SMs.  Without a spiral
+// (PLAIN) the flutter depends on the azimuth alone, which is known ahead: two
+// evaluations a step instead of four, their cells loaded a step before.
+// 1280 tracks of 523 steps: 1.37 -> 0.40 ms (2.5 ms before field64);
+// 100000 tracks of 128 steps: 1.40 -> 0.29 ms.
+template <bool PLAIN>
+__global__ void __launch_bounds__(32) theta_track_kernel(const __grid_constant__ FieldK f,
                                                          const __grid_constant__ ffa_theta_track_desc d)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.m) return;
     double x[4] = {d.x0[5 * i], d.x0[5 * i + 1], d.x0[5 * i + 2], d.x0[5 * i + 3]};
-    const double P = d.x0[5 * i + 4], q = d.q;
+    const double qP = d.q / d.x0[5 * i + 4];
     const double h = d.t_end / (double)(d.n_points - 1);
     const int nc = d.traj_cols;
     double *tr = d.traj ? d.traj + (int64_t)i * d.n_points * nc : nullptr;
@@ -1571,26 +1626,57 @@ __global__ void __launch_bounds__(64) theta_track_kernel(const __grid_constant__
         if (nc == 7) {
             row[2] = x[2];
             row[3] = x[3];
-            const double fim = fmod(fmod(ts, 2.0 * PI), f.period);
             int clamped = 0;
-            field64<0>(f, x[0], 1.0 / x[0], fim, x[2], row[4], row[5], row[6], clamped);
+            field64<0>(f, x[0], 1.0 / x[0], sector_azimuth(f, ts), x[2], row[4], row[5], row[6], clamped);
         }
     };
     if (tr) record(0, 0.0);
+    auto start = [&](int s) { return d.time_mode == 0 ? (double)s * h : t; };
+    // PLAIN: the flutter at the step's start, and the cells of its middle and
+    // end (the next step's start)
+    double F0 = 0.0, Fp0 = 0.0;
+    FlutterCell mid, end;
+    if constexpr (PLAIN) {
+        flutter_eval(f, flutter_fetch(f, sector_azimuth(f, 0.0)), F0, Fp0);
+        mid = flutter_fetch(f, sector_azimuth(f, 0.5 * h));
+        end = flutter_fetch(f, sector_azimuth(f, h));
+    }
     for (int s = 0; s < d.n_points - 1; ++s) {
-        if (d.time_mode == 0) t = (double)s * h;
-        double k1[4], k2[4], k3[4], k4[4], y[4], dd[4];
-        seo_rhs(f, t, x, P, q, dd);
-        for (int c = 0; c < 4; ++c) { k1[c] = h * dd[c]; y[c] = x[c] + 0.5 * k1[c]; }
-        seo_rhs(f, t + 0.5 * h, y, P, q, dd);
-        for (int c = 0; c < 4; ++c) { k2[c] = h * dd[c]; y[c] = x[c] + 0.5 * k2[c]; }
-        seo_rhs(f, t + 0.5 * h, y, P, q, dd);
-        for (int c = 0; c < 4; ++c) { k3[c] = h * dd[c]; y[c] = x[c] + k3[c]; }
-        seo_rhs(f, t + h, y, P, q, dd);
-        for (int c = 0; c < 4; ++c) {
-            k4[c] = h * dd[c];
-            x[c] = x[c] + (k1[c] + 2 * k2[c] + 2 * k3[c] + k4[c]) / 6;
+        t = start(s);
+        double F1 = 0.0, Fp1 = 0.0, F2 = 0.0, Fp2 = 0.0;
+        if constexpr (PLAIN) {
+            flutter_eval(f, mid, F1, Fp1);
+            flutter_eval(f, end, F2, Fp2);
+            const double tn = d.time_mode == 0 ? (double)(s + 1) * h : t + h;
+            mid = flutter_fetch(f, sector_azimuth(f, tn + 0.5 * h));
+            end = flutter_fetch(f, sector_azimuth(f, tn + h));
         }
+        auto rhs = [&](double ts, const double *y, double F, double Fp, double *k) {
+            if constexpr (PLAIN) {
+                const double G = power_eval(f, power_fetch(f, y[0]), y[0]);
+                seo_rhs(y, qP, F, Fp, G, f.k * G, 0.0, k);
+            } else {
+                const Tables tab = tables_fetch(f, y[0], sector_azimuth(f, ts));
+                double G, kG;
+                tables_eval(f, tab, y[0], F, Fp, G, kG);
+                seo_rhs(y, qP, F, Fp, G, kG, tab.spiral_p, k);
+            }
+        };
+        double y[4], k[4], S[4];
+        rhs(t, x, F0, Fp0, k);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { S[c] = k[c]; y[c] = fma(0.5 * h, k[c], x[c]); }
+        rhs(t + 0.5 * h, y, F1, Fp1, k);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { S[c] = fma(2.0, k[c], S[c]); y[c] = fma(0.5 * h, k[c], x[c]); }
+        rhs(t + 0.5 * h, y, F1, Fp1, k);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { S[c] = fma(2.0, k[c], S[c]); y[c] = fma(h, k[c], x[c]); }
+        rhs(t + h, y, F2, Fp2, k);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) x[c] = fma(h * (1.0 / 6.0), S[c] + k[c], x[c]);
+        F0 = F2;
+        Fp0 = Fp2;
         if (d.time_mode != 0) t = t + h;
         if (tr) record(s + 1, d.time_mode != 0 ? t : (double)(s + 1) * h);
     }
@@ -1599,7 +1685,9 @@ __global__ void __launch_bounds__(64) theta_track_kernel(const __grid_constant__
 
 cudaError_t launch_theta_track(const FieldK &f, const ffa_theta_track_desc &d, cudaStream_t s)
 {
-    theta_track_kernel<<<(unsigned)((d.m + 63) / 64), 64, 0, s>>>(f, d);
+    const unsigned g = (unsigned)((d.m + 31) / 32);
+    if (f.spiral_zero && !f.unusual) theta_track_kernel<true><<<g, 32, 0, s>>>(f, d);
+    else theta_track_kernel<false><<<g, 32, 0, s>>>(f, d);
     return cudaGetLastError();
 }
 

@@ -81,3 +81,36 @@ def test_one_step_matches_oracle(fringe, k, dr, solver):
         assert np.max(np.abs(got[:, c] - ref[:, c]) / np.maximum(np.abs(ref[:, c]), 1e-3)) < 1e-14, c
     for c in (1, 2, 3):
         assert np.max(np.abs(got[:, c] - ref[:, c])) < 1e-14 * np.abs(ref[:, c]).max(), c
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("fringe,m,turns", [(1.17, 1, 1 / 12), (1.17, 33, 2.05), (0.002, 33, 1 / 12)])
+def test_azimuth_tracks_match_oracle(fringe, m, turns, mode):
+    """Tracks without a spiral (the flutter taken a step ahead; with the
+    sharp fringe evaluated directly) over a sector and past two turns, both
+    stage-azimuth rules, with the trajectory and its field.  Tolerance: the
+    1e-12 per sector of the spiral lattice's test."""
+    import warnings
+    from oracle import oracle as O
+    from pyffa_b200 import seo, synthetic
+    from pyffa_b200.constants import FFAG_ConversionTools, Q
+    from pyffa_b200.fields import FFAG_Bfield_analytical
+    cfg = synthetic.lattice_bmap(r_range=(8.0, 9.3, 0.01), theta_step_deg=0.05)
+    cfg["Bmap"]["fringe_width_1"] = [0, fringe, 0, fringe, 0]
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        bm = FFAG_Bfield_analytical(config=cfg, max_order=0, AddNumricalMap=False)
+    rng = np.random.default_rng(9)
+    x0 = np.zeros((m, 5))
+    x0[:, 0] = 8.13 + 1e-3 * rng.standard_normal(m)
+    x0[:, 1] = 0.1168 + 1e-3 * rng.standard_normal(m)
+    x0[:, 2:4] = 1e-3 * rng.standard_normal((m, 2))
+    x0[:, 4] = FFAG_ConversionTools().Ek2P(300.0 + rng.random(m))
+    t_end, cols = 2 * np.pi * turns, 7
+    g1, gt, _ = seo.ThetaTracker(bm, Q).run(x0, t_end, 0.001, mode, True, cols)
+    o1, ot, _ = O.ThetaTracker(bm, Q).run(x0, t_end, 0.001, mode, True, cols)
+    tol = 1e-12 * max(1.0, 12 * turns)
+    for c in range(4):
+        assert np.abs(g1[:, c] - o1[:, c]).max() <= tol * np.abs(ot[..., c]).max(), c
+    for c in range(cols):
+        assert np.abs(gt[..., c] - ot[..., c]).max() <= tol * np.abs(ot[..., c]).max(), c
