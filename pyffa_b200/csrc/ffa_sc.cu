@@ -18,7 +18,8 @@
 //           (DistributeChargeSBS_Njit :244-312 accumulates float32 in
 //           particle order)
 //   green   open boundary only: the transform of the free-space Green's
-//           function on the doubled grid, float64, as a sum of cosines
+//           function on the doubled grid, float64, as a sum of cosines (rows
+//           beside the deposit, columns after it)
 //   solve   ONE block per slice, the slice resident in shared memory: real
 //           FFT of the charge (rows paired as real and imaginary parts),
 //           per column the z transform, the kernel multiply (periodic
@@ -51,10 +52,11 @@ constexpr int SC_TB = 256;
 constexpr int SC_BLOCKS = 444;             // pass1: 3 per SM on 148 SMs (one wave); fixed for determinism
 constexpr double FIX_SCALE = 1099511627776.0;  // 2^40
 constexpr double EPS0 = 8.854187817e-12;
+constexpr int64_t SEO_CELLS_MAX = 1 << 16;     // closed-orbit cells a plan packs (4 MB)
 
 struct SCState {
     ffa_sc_diag diag;
-    double inv_dx, inv_dz;
+    double inv_dx, inv_dz, inv_step;   // of the cell sizes and the slice width
     int32_t degenerate;   // dx <= 0 or dz <= 0: fields are not updated
     int32_t bad;          // degenerate or bunch length <= 0: gathered field = 0
 };
@@ -67,26 +69,65 @@ struct Partial {
     long long count;
 };
 
-__device__ __forceinline__ double fast_mod(double a, double b) { return a - b * floor(a / b); }
+// The kernels of an update follow one another by programmatic dependent launch:
+// each starts as the blocks of its predecessor exit and waits for its results
+// before it touches memory (chain_wait, no effect on an ordinary launch).
+// Letting a successor start earlier (griddepcontrol.launch_dependents) cost
+// 10-20 us of 145: its waiting blocks take the room of the running ones.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ double py_mod(double a, double b)
 {
-    double r = fmod(a, b);
+    // fmod: the remainder of the truncated quotient is exact; a quotient that
+    // rounded up to the next integer leaves it with the wrong sign
+    double n = trunc(a / b), r = fma(-n, b, a);
+    if (r != 0.0 && ((r < 0.0) != (a < 0.0))) r = fma(-(n - copysign(1.0, n)), b, a);
     if (r != 0.0 && ((r < 0.0) != (b < 0.0))) r += b;
     return r;
 }
 
-// Bilinear_interp_2D_vect_uniform (src/FFAG_MathTools.py:828-936) for one point
-__device__ __forceinline__ double seo_lookup(const double *Z, double X0, double dX, int64_t NX, double Y0,
-                                             double dY, int64_t NY, double x, double y)
+// a / d for a divisor known in advance, inv = 1 / d rounded: the quotient
+// estimate and one correction by its exact residual give the correctly rounded
+// quotient (Markstein; Brisebarre, Muller and Raina, "Accelerating correctly
+// rounded floating-point division when the divisor is known in advance"), in
+// three operations without a branch.  Infinite a give NaN.
+struct Divisor {
+    double d, inv;
+    __host__ __device__ Divisor(double d_, double inv_) : d(d_), inv(inv_) {}
+    __device__ double quotient(double a) const
+    {
+        const double q = a * inv;
+        return fma(fma(-q, d, a), inv, q);
+    }
+};
+
+// the update's constant divisors
+struct Divisors {
+    Divisor turn, cc, e0, dE, df;
+    explicit Divisors(const ffa_sc_desc &d)
+        : turn(2 * PI, 1.0 / (2 * PI)), cc(d.speed_c * d.speed_c, 1.0 / (d.speed_c * d.speed_c)),
+          e0(d.E0_J, 1.0 / d.E0_J), dE(d.dEk, 1.0 / d.dEk), df(d.dfi, 1.0 / d.dfi) {}
+};
+
+// The four corners of one closed-orbit table cell: (r0, pr0) at (i, j),
+// (i, j + 1), (i + 1, j), (i + 1, j + 1), two 32-byte loads
+struct __align__(32) SeoCell {
+    double r00, p00, r01, p01, r10, p10, r11, p11;
+};
+
+__device__ __forceinline__ SeoCell seo_cell(const ffa_sc_desc &d, int i, int j)
 {
-    int64_t i = (int64_t)floor((x - X0) / dX);
-    int64_t j = (int64_t)floor((y - Y0) / dY);
-    if (i < 0) i = 0; else if (i >= NX - 1) i = NX - 2;
-    if (j < 0) j = 0; else if (j >= NY - 1) j = NY - 2;
-    const double tx = (x - (X0 + (double)i * dX)) / dX, ty = (y - (Y0 + (double)j * dY)) / dY;
-    const double z00 = Z[i * NY + j], z01 = Z[i * NY + j + 1], z10 = Z[(i + 1) * NY + j], z11 = Z[(i + 1) * NY + j + 1];
-    return (1 - tx) * (1 - ty) * z00 + (1 - tx) * ty * z01 + tx * (1 - ty) * z10 + tx * ty * z11;
+    const double *R = d.seo_r + (int64_t)i * d.nfi + j, *P = d.seo_pr + (int64_t)i * d.nfi + j;
+    return {R[0], P[0], R[1], P[1], R[d.nfi], P[d.nfi], R[d.nfi + 1], P[d.nfi + 1]};
+}
+
+__device__ __forceinline__ SeoCell load_cell(const SeoCell *c)
+{
+    SeoCell v;
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.r00), "=d"(v.p00), "=d"(v.r01), "=d"(v.p01) : "l"(c));
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.r10), "=d"(v.p10), "=d"(v.r11), "=d"(v.p11)
+        : "l"(reinterpret_cast<const double *>(c) + 4));
+    return v;
 }
 
 // Warp tree (shuffle down) then warp 0's values folded in warp order by
@@ -103,13 +144,14 @@ struct OpMin { __device__ double operator()(double a, double b) const { return f
 struct OpMax { __device__ double operator()(double a, double b) const { return fmax(a, b); } };
 
 // Block reduction of one Partial per thread (valid in thread 0).  Per value:
-// warp tree, then thread 0 folds the warps' results starting from the
-// identity (0, +1e300 / -1e300 for min / max), in warp order.
+// warp tree, then the warps' results folded starting from the identity (0,
+// +1e300 / -1e300 for min / max), in warp order, one lane per value.
 __device__ Partial block_partial(const Partial &p)
 {
     constexpr int NW = SC_TB / 32;
     __shared__ double sh[NW][13];
     __shared__ long long shc[NW];
+    __shared__ Partial res;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     double v[13];
     v[0] = warp_fold(p.sum_gamma, OpSum());
@@ -128,21 +170,21 @@ __device__ Partial block_partial(const Partial &p)
         shc[w] = c;
     }
     __syncthreads();
-    Partial r;
-    r.sum_gamma = 0.0; r.sx = r.sz = r.sx2 = r.sz2 = 0.0; r.count = 0;
-    for (int k = 0; k < 4; ++k) { r.amin[k] = 1e300; r.amax[k] = -1e300; }
-    if (threadIdx.x == 0) {
-        for (int q = 0; q < NW; ++q) {
-            r.sum_gamma += sh[q][0];
-            for (int k = 0; k < 4; ++k) {
-                r.amin[k] = fmin(r.amin[k], sh[q][1 + k]);
-                r.amax[k] = fmax(r.amax[k], sh[q][5 + k]);
-            }
-            r.sx += sh[q][9]; r.sz += sh[q][10]; r.sx2 += sh[q][11]; r.sz2 += sh[q][12];
-            r.count += shc[q];
-        }
+    const int k = threadIdx.x;
+    if (k < 13) {
+        const bool mn = k >= 1 && k < 5, mx = k >= 5 && k < 9;
+        double t = mn ? 1e300 : (mx ? -1e300 : 0.0);
+        for (int q = 0; q < NW; ++q) t = mn ? fmin(t, sh[q][k]) : (mx ? fmax(t, sh[q][k]) : t + sh[q][k]);
+        double *out = k == 0 ? &res.sum_gamma : (mn ? res.amin + (k - 1) : (mx ? res.amax + (k - 5)
+                      : (k == 9 ? &res.sx : (k == 10 ? &res.sz : (k == 11 ? &res.sx2 : &res.sz2)))));
+        *out = t;
+    } else if (k == 13) {
+        long long t = 0;
+        for (int q = 0; q < NW; ++q) t += shc[q];
+        res.count = t;
     }
-    return r;
+    __syncthreads();
+    return res;
 }
 
 // The final state from the block partials, by one block: each thread folds a
@@ -179,6 +221,7 @@ __device__ void finalize_state(const Partial *part, int nblk, const ffa_sc_desc 
     D.fi_s = fi_s;
     D.fi_e = fi_e;
     D.slice_step = (fi_e - fi_s) / (d.ns - 1);
+    st->inv_step = 1.0 / D.slice_step;
     D.count = cnt;
     D.mean_gamma_m1 = cnt > 0 ? t.sum_gamma / (double)cnt - 1.0 : 0.0;
     // box from the moments
@@ -223,13 +266,35 @@ __device__ void finalize_state(const Partial *part, int nblk, const ffa_sc_desc 
 
 // ----------------------------------------------------------------- passes
 
+// Before the update: clears the charge accumulator (and the block counter
+// after it) and packs the closed-orbit tables by cell when `cells` is given.
+__global__ void __launch_bounds__(SC_TB) sc_prepare(ffa_sc_desc d, int64_t words, unsigned long long *acc, SeoCell *cells)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t e = t; e < words / 2; e += nt) reinterpret_cast<ulonglong2 *>(acc)[e] = make_ulonglong2(0, 0);
+    if (t == 0 && (words & 1)) acc[words - 1] = 0;
+    if (!cells) return;
+    const int nj = (int)d.nfi - 1, nc = ((int)d.nE - 1) * nj;
+    for (int c = (int)t; c < nc; c += (int)nt) cells[c] = seo_cell(d, c / nj, c % nj);
+}
+
 // `done` counts finished blocks; it must be zero at launch (it sits in the
 // slot after the charge accumulator, which is cleared before every update).
-__global__ void __launch_bounds__(SC_TB, 3) sc_pass1(ffa_state_soa S, int64_t n, ffa_sc_desc d, double *x_out,
-                                                     double *pr0_out, Partial *part, unsigned long long *done,
-                                                     SCState *st, int64_t *status)
+//
+// The particles of a warp sit in as many table cells, and a warp load costs
+// the L1 data pipe a cycle per line it touches: eight separate table reads
+// cost 8 x 32, the packed cell (`cells`, sc_prepare) 2 x 32.  That and the
+// fourteen divisions by constants were the pass's time; the sums keep their
+// order and every value its rounding.  1e6 particles: 37.7 -> 31.5 us; now bound by
+// the latency of the state and table loads at 24 warps per SM.
+__global__ void __launch_bounds__(SC_TB, 3) sc_pass1(ffa_state_soa S, int64_t n, ffa_sc_desc d,
+                                                     const Divisors by, const SeoCell *__restrict__ cells, double *x_out, double *pr0_out,
+                                                     Partial *part, unsigned long long *done, SCState *st,
+                                                     int64_t *status)
 {
+    chain_wait();
     const double shifts[4] = {0.0, PI, PI * 0.5, PI * 1.5};
+    const int nE = (int)d.nE, nfi = (int)d.nfi;
     Partial p;
     p.sum_gamma = 0.0; p.sx = p.sz = p.sx2 = p.sz2 = 0.0; p.count = 0;
     for (int k = 0; k < 4; ++k) { p.amin[k] = 1e30; p.amax[k] = -1e30; }
@@ -239,21 +304,31 @@ __global__ void __launch_bounds__(SC_TB, 3) sc_pass1(ffa_state_soa S, int64_t n,
         if (d.boris) {
             const double rd = r * f5;
             const double v2 = vr * vr + vz * vz + rd * rd;
-            g = 1.0 / sqrt(1.0 - v2 / (d.speed_c * d.speed_c));
+            g = 1.0 / sqrt(1.0 - by.cc.quotient(v2));
         } else {
-            g = f5 / d.E0_J;
+            g = by.e0.quotient(f5);
         }
-        const double fm = fi - 2 * PI * floor(fi / (2 * PI));
+        const double fm = fi - 2 * PI * floor(by.turn.quotient(fi));
         const double Ek = (g - 1) * d.E0_rest_MeV;
-        const double r0 = seo_lookup(d.seo_r, d.Ek0, d.dEk, d.nE, d.fi0, d.dfi, d.nfi, Ek, fm);
-        pr0_out[i] = seo_lookup(d.seo_pr, d.Ek0, d.dEk, d.nE, d.fi0, d.dfi, d.nfi, Ek, fm);
+        // Bilinear_interp_2D_vect_uniform (src/FFAG_MathTools.py:828-936) of
+        // r0 and pr0 (indices saturate outside the int range, where they are
+        // clamped anyway)
+        int a = (int)floor(by.dE.quotient(Ek - d.Ek0)), b = (int)floor(by.df.quotient(fm - d.fi0));
+        a = a < 0 ? 0 : (a >= nE - 1 ? nE - 2 : a);
+        b = b < 0 ? 0 : (b >= nfi - 1 ? nfi - 2 : b);
+        const SeoCell c = cells ? load_cell(cells + (int64_t)a * (nfi - 1) + b) : seo_cell(d, a, b);
+        const double tx = by.dE.quotient(Ek - (d.Ek0 + (double)a * d.dEk)), ty = by.df.quotient(fm - (d.fi0 + (double)b * d.dfi));
+        const double r0 = (1 - tx) * (1 - ty) * c.r00 + (1 - tx) * ty * c.r01 + tx * (1 - ty) * c.r10 + tx * ty * c.r11;
+        pr0_out[i] = (1 - tx) * (1 - ty) * c.p00 + (1 - tx) * ty * c.p01 + tx * (1 - ty) * c.p10 + tx * ty * c.p11;
         const double xi = r - r0, zi = z;
         x_out[i] = xi;
         p.sum_gamma += g;
         ++p.count;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const double v = fast_mod(fm + shifts[k], 2 * PI);
+            // (fm + shift) mod 2 pi, below 4 pi
+            double v = fm + shifts[k];
+            if (v >= 2 * PI) v -= 2 * PI;
             p.amin[k] = fmin(p.amin[k], v);
             p.amax[k] = fmax(p.amax[k], v);
         }
@@ -281,55 +356,6 @@ __global__ void __launch_bounds__(SC_TB, 3) sc_pass1(ffa_state_soa S, int64_t n,
     finalize_state(part, gridDim.x, d, st, status);
 }
 
-// slice index of every live particle (-1 otherwise), then the CIC deposit.
-// The integer sums do not depend on the order of the atomics, so any grid
-// gives the same cube; two particles per pass keep two particles' loads in
-// flight per thread.
-__global__ void __launch_bounds__(SC_TB) sc_deposit(ffa_state_soa S, int64_t n, ffa_sc_desc d, const double *x,
-                                                    int32_t *slice, int64_t *cell, const SCState *st,
-                                                    unsigned long long *acc)
-{
-    const int bad = st->bad;
-    const double fi_s = st->diag.fi_s, step = st->diag.slice_step;
-    const double xmin = st->diag.xmin, zmin = st->diag.zmin, inv_dx = st->inv_dx, inv_dz = st->inv_dz;
-    const int nx = d.nx, nz = d.nz;
-    auto one = [&](int64_t i, uint8_t alive, double fi, double xi, double zi) {
-        if (alive == 0) {
-            slice[i] = -1;
-            cell[i] = -1;
-            return;
-        }
-        fi = fi - 2 * PI * floor(fi / (2 * PI));
-        if (fi < fi_s) fi += 2 * PI;
-        int64_t s = (int64_t)((fi - fi_s) / step);
-        if (s < 0) s = 0; else if (s >= d.ns) s = d.ns - 1;
-        slice[i] = (int32_t)s;
-        if (bad) {
-            cell[i] = -1;
-            return;
-        }
-        const double rx = (xi - xmin) * inv_dx, rz = (zi - zmin) * inv_dz;
-        int64_t ix = (int64_t)floor(rx), iz = (int64_t)floor(rz);
-        double fx = rx - (double)ix, fz = rz - (double)iz;
-        if (ix < 0) { ix = 0; fx = 0.0; } else if (ix >= nx - 1) { ix = nx - 2; fx = 1.0; }
-        if (iz < 0) { iz = 0; fz = 0.0; } else if (iz >= nz - 1) { iz = nz - 2; fz = 1.0; }
-        const int64_t c0 = (s * nz + iz) * nx + ix;
-        cell[i] = c0;
-        atomicAdd(acc + c0, (unsigned long long)llrint((1.0 - fx) * (1.0 - fz) * FIX_SCALE));
-        atomicAdd(acc + c0 + 1, (unsigned long long)llrint(fx * (1.0 - fz) * FIX_SCALE));
-        atomicAdd(acc + c0 + nx, (unsigned long long)llrint((1.0 - fx) * fz * FIX_SCALE));
-        atomicAdd(acc + c0 + nx + 1, (unsigned long long)llrint(fx * fz * FIX_SCALE));
-    };
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 2 * stride) {
-        const int64_t k = i + stride < n ? i + stride : i;
-        const uint8_t a0 = S.surv[i], a1 = S.surv[k];
-        const double f0 = S.fi[i], f1 = S.fi[k], x0 = x[i], x1 = x[k], z0 = S.z[i], z1 = S.z[k];
-        one(i, a0, f0, x0, z0);
-        if (k != i) one(k, a1, f1, x1, z1);
-    }
-}
-
 // --------------------------------------------------- open-boundary Green's
 //
 // G(x, z) = -ln(x^2 + z^2) / (4 pi eps0) on the doubled (NZ, NX) grid with
@@ -355,90 +381,131 @@ __device__ __forceinline__ double green_point(int j, int i, double dx, double dz
     return v * dx * dz;
 }
 
-// Both sums are small dense products, (hz + 1) x (hx + 1) outputs of
-// hx + 1 (rows) or hz + 1 (columns) terms, tiled: a block computes 32 x 32
-// outputs (each thread one kx and four rows j or kz), with the shared
-// operand staged in GT-term chunks through shared memory and the cosine
-// table of the summed axis in shared memory; every output is summed over
-// increasing i (or j) as one chain of multiply-adds.
-constexpr int GT = 64;
+// Both sums are small dense products, (hz + 1) x (hx + 1) outputs of hx + 1
+// (rows) or hz + 1 (columns) terms, each output one chain of multiply-adds over
+// increasing i (or j).  They are cut for latency: one block per row j (or
+// column kx), one thread per output, the row and the cosine table in shared
+// memory.  The rows are the first blocks of the deposit's launch, which does
+// not need them, the columns a launch of their own after it.  128 x 128 cells
+// (256 x 256 doubled): points, rows and columns in 32 x 32 tiles took 33 us on
+// 25 blocks (longer than the deposit they ran beside, and the second stream's
+// events cost some 15 us), rows and columns now 6 and 7 us.
+constexpr int GREEN_TB = 256;
 
-// w_i G[j][i] over the first quadrant (j <= NZ/2, i <= NX/2), row-major,
-// every point once
-__global__ void __launch_bounds__(256) sc_green_points(int NZ, int NX, const SCState *st, double *G)
+// T[j][.] of row j by one block: w_i G[j][i] of the row, then its cosine sums
+// (the cosines before the wait for the kernel before)
+__device__ __forceinline__ void green_row(int j, int NX, const SCState *st, double *T)
 {
+    extern __shared__ double green_sm[];     // w_i G[j][i] (hx + 1), cos(2 pi m / NX) (NX)
+    const int hx = NX / 2;
+    double *g = green_sm, *cx = green_sm + hx + 1;
+    for (int m = threadIdx.x; m < NX; m += GREEN_TB) cx[m] = cospi(2.0 * (double)m / (double)NX);
+    chain_wait();
     if (st->bad) return;
-    const int hx = NX / 2, hz = NZ / 2;
     const double dx = st->diag.dx, dz = st->diag.dz;
-    const int64_t tot = (int64_t)(hz + 1) * (hx + 1);
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
-        const int j = (int)(e / (hx + 1)), i = (int)(e - (int64_t)j * (hx + 1));
-        G[e] = ((i == 0 || i == hx) ? 1.0 : 2.0) * green_point(j, i, dx, dz);
+    for (int i = threadIdx.x; i <= hx; i += GREEN_TB) g[i] = ((i == 0 || i == hx) ? 1.0 : 2.0) * green_point(j, i, dx, dz);
+    __syncthreads();
+    for (int kx = threadIdx.x; kx <= hx; kx += GREEN_TB) {
+        double a = 0.0;
+#pragma unroll 8
+        for (int i = 0; i <= hx; ++i) a += g[i] * cx[(i * kx) & (NX - 1)];
+        T[(int64_t)j * (hx + 1) + kx] = a;
     }
 }
 
-__global__ void __launch_bounds__(256) sc_green_rows(int NZ, int NX, const SCState *st, const double *G, double *T)
+// gk[.][kx] of column kx = blockIdx.x
+__global__ void __launch_bounds__(GREEN_TB) sc_green_cols(int NZ, int NX, const SCState *st, const double *T, float *gk)
 {
+    extern __shared__ double green_sm[];     // w_j T[j][kx] (hz + 1), cos(2 pi m / NZ) (NZ)
+    const int hx = NX / 2, hz = NZ / 2, kx = blockIdx.x;
+    double *t = green_sm, *cz = green_sm + hz + 1;
+    for (int m = threadIdx.x; m < NZ; m += GREEN_TB) cz[m] = cospi(2.0 * (double)m / (double)NZ);
+    chain_wait();
     if (st->bad) return;
-    __shared__ double g[GT][33];     // w_i G[j][i] for a chunk of i and the block's 32 rows j (padded)
-    extern __shared__ double cx[];   // cos(2 pi m / NX), m < NX
-    const int hx = NX / 2, hz = NZ / 2;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int kx = blockIdx.x * 32 + tx, jb = blockIdx.y * 32;
-    for (int m = threadIdx.x; m < NX; m += blockDim.x) cx[m] = cospi(2.0 * (double)m / (double)NX);
-    double a[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int i0 = 0; i0 <= hx; i0 += GT) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < GT * 32; e += blockDim.x) {
-            const int ii = e & (GT - 1), jj = e / GT, i = i0 + ii, j = jb + jj;
-            g[ii][jj] = (i <= hx && j <= hz) ? G[(int64_t)j * (hx + 1) + i] : 0.0;
-        }
-        __syncthreads();
-        const int in = min(GT, hx + 1 - i0);
-        for (int ii = 0; ii < in; ++ii) {
-            const double c = cx[((i0 + ii) * kx) & (NX - 1)];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) a[q] += g[ii][ty * 4 + q] * c;
-        }
-    }
-    if (kx > hx) return;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int j = jb + ty * 4 + q;
-        if (j <= hz) T[(int64_t)j * (hx + 1) + kx] = a[q];
+    for (int j = threadIdx.x; j <= hz; j += GREEN_TB) t[j] = ((j == 0 || j == hz) ? 1.0 : 2.0) * T[(int64_t)j * (hx + 1) + kx];
+    __syncthreads();
+    for (int kz = threadIdx.x; kz <= hz; kz += GREEN_TB) {
+        double a = 0.0;
+#pragma unroll 8
+        for (int j = 0; j <= hz; ++j) a += t[j] * cz[(j * kz) & (NZ - 1)];
+        gk[(int64_t)kz * (hx + 1) + kx] = (float)a;
     }
 }
 
-__global__ void __launch_bounds__(256) sc_green_cols(int NZ, int NX, const SCState *st, const double *T, float *gk)
+// ----------------------------------------------------------------- deposit
+
+// slice index of every live particle (-1 otherwise), then the CIC deposit.
+// The integer sums do not depend on the order of the atomics, so any grid
+// gives the same cube; two particles per pass keep two particles' loads in
+// flight per thread.
+//
+// A warp's atomics cost a cycle of the load/store pipe per line they touch and
+// an L2 operation per sector.  The two charges of a particle in one row are
+// neighbours, so a pair of lanes adds both in one instruction, first the even
+// lane's particle, then the odd one's: 16 lines per instruction instead of 32,
+// and one L2 operation for both where they share a sector (three times in
+// four).  1e6 particles: 42.0 -> 24.4 us.
+__global__ void __launch_bounds__(SC_TB) sc_deposit(ffa_state_soa S, int64_t n, ffa_sc_desc d, const double *x,
+                                                    int32_t *slice, int64_t *cell, const SCState *st,
+                                                    unsigned long long *acc, int rows, int NX, double *T)
 {
-    if (st->bad) return;
-    __shared__ double t[GT][32];     // w_j T[j][kx] for a chunk of j and the block's 32 columns kx
-    extern __shared__ double cz[];   // cos(2 pi m / NZ), m < NZ
-    const int hx = NX / 2, hz = NZ / 2;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int kx = blockIdx.x * 32 + tx, kzb = blockIdx.y * 32 + ty * 4;
-    for (int m = threadIdx.x; m < NZ; m += blockDim.x) cz[m] = cospi(2.0 * (double)m / (double)NZ);
-    double a[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int j0 = 0; j0 <= hz; j0 += GT) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < GT * 32; e += blockDim.x) {
-            const int jj = e >> 5, xx = e & 31, j = j0 + jj, x = blockIdx.x * 32 + xx;
-            t[jj][xx] = (j <= hz && x <= hx) ? ((j == 0 || j == hz) ? 1.0 : 2.0) * T[(int64_t)j * (hx + 1) + x] : 0.0;
-        }
-        __syncthreads();
-        const int jn = min(GT, hz + 1 - j0);
-        for (int jj = 0; jj < jn; ++jj) {
-            const double v = t[jj][tx];
-            const int j = j0 + jj;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) a[q] += v * cz[(j * (kzb + q)) & (NZ - 1)];
-        }
+    if ((int)blockIdx.x < rows) {            // open boundary: one row of the Green transform
+        green_row(blockIdx.x, NX, st, T);
+        return;
     }
-    if (kx > hx) return;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int kz = kzb + q;
-        if (kz <= hz) gk[(int64_t)kz * (hx + 1) + kx] = (float)a[q];
+    chain_wait();
+    const int64_t block = (int64_t)blockIdx.x - rows;
+    const int bad = st->bad;
+    const double fi_s = st->diag.fi_s;
+    const Divisor turn(2 * PI, 1.0 / (2 * PI)), step(st->diag.slice_step, st->inv_step);
+    const double xmin = st->diag.xmin, zmin = st->diag.zmin, inv_dx = st->inv_dx, inv_dz = st->inv_dz;
+    const int nx = d.nx, nz = d.nz;
+    const int odd = threadIdx.x & 1;
+    // every lane of the warp comes here
+    auto one = [&](int64_t i, bool valid, uint8_t alive, double fi, double xi, double zi) {
+        int64_t c0 = -1;
+        unsigned long long w00 = 0, w01 = 0, w10 = 0, w11 = 0;   // row z, column x
+        if (valid) {
+            int s = -1;
+            if (alive != 0) {
+                fi = fi - 2 * PI * floor(turn.quotient(fi));
+                if (fi < fi_s) fi += 2 * PI;
+                s = (int)step.quotient(fi - fi_s);
+                if (s < 0) s = 0; else if (s >= d.ns) s = d.ns - 1;
+                if (!bad) {
+                    const double rx = (xi - xmin) * inv_dx, rz = (zi - zmin) * inv_dz;
+                    int ix = (int)floor(rx), iz = (int)floor(rz);
+                    double fx = rx - (double)ix, fz = rz - (double)iz;
+                    if (ix < 0) { ix = 0; fx = 0.0; } else if (ix >= nx - 1) { ix = nx - 2; fx = 1.0; }
+                    if (iz < 0) { iz = 0; fz = 0.0; } else if (iz >= nz - 1) { iz = nz - 2; fz = 1.0; }
+                    c0 = ((int64_t)s * nz + iz) * nx + ix;
+                    w00 = (unsigned long long)llrint((1.0 - fx) * (1.0 - fz) * FIX_SCALE);
+                    w01 = (unsigned long long)llrint(fx * (1.0 - fz) * FIX_SCALE);
+                    w10 = (unsigned long long)llrint((1.0 - fx) * fz * FIX_SCALE);
+                    w11 = (unsigned long long)llrint(fx * fz * FIX_SCALE);
+                }
+            }
+            slice[i] = s;
+            cell[i] = c0;
+        }
+        // each lane gets its partner's cell and the two charges it adds for it
+        const int64_t cp = __shfl_xor_sync(0xffffffffu, c0, 1);
+        const unsigned long long a = __shfl_xor_sync(0xffffffffu, odd ? w00 : w01, 1);
+        const unsigned long long b = __shfl_xor_sync(0xffffffffu, odd ? w10 : w11, 1);
+        const int64_t ce = odd ? cp : c0, co = odd ? c0 : cp;
+        if (ce >= 0) atomicAdd(acc + ce + odd, odd ? a : w00);
+        if (co >= 0) atomicAdd(acc + co + odd, odd ? w01 : a);
+        if (ce >= 0) atomicAdd(acc + ce + nx + odd, odd ? b : w10);
+        if (co >= 0) atomicAdd(acc + co + nx + odd, odd ? w11 : b);
+    };
+    const int64_t stride = ((int64_t)gridDim.x - rows) * blockDim.x;
+    for (int64_t base = block * blockDim.x; base < n; base += 2 * stride) {
+        const int64_t i = base + threadIdx.x, k = i + stride;
+        const int64_t li = i < n ? i : n - 1, lk = k < n ? k : n - 1;
+        const uint8_t a0 = S.surv[li], a1 = S.surv[lk];
+        const double f0 = S.fi[li], f1 = S.fi[lk], x0 = x[li], x1 = x[lk], z0 = S.z[li], z1 = S.z[lk];
+        one(i, i < n, a0, f0, x0, z0);
+        if (base + stride < n) one(k, k < n, a1, f1, x1, z1);   // the same for the whole block
     }
 }
 
@@ -462,7 +529,11 @@ template <> struct Split<64> { static constexpr int N1 = 8, N2 = 8; };
 template <> struct Split<128> { static constexpr int N1 = 8, N2 = 16; };
 template <> struct Split<256> { static constexpr int N1 = 16, N2 = 16; };
 
-constexpr int SOLVE_TB = 512;
+// Threads of the fused solve: 512, and 544 for the 256 x 256 doubled grid,
+// whose 65 columns per CTA then take two passes of 34 line groups instead of
+// three of 32 (the third with a single column): 45.7 -> 41.0 us.
+template <int NX>
+constexpr int solve_tb = NX == 256 ? 544 : 512;
 
 // group scratch stride (float2): N2 rows of N1 + 1, padded so that the
 // groups sharing a half-warp land on disjoint banks
@@ -613,8 +684,20 @@ constexpr size_t solve_smem()
     constexpr int P = NX / 2 + 1;
     constexpr int SX = scratch_stride<Split<NX>::N1, Split<NX>::N2>();
     constexpr int SZ = scratch_stride<Split<NZ>::N1, Split<NZ>::N2>();
-    constexpr int GX = SOLVE_TB / Split<NX>::N1 * SX, GZ = SOLVE_TB / Split<NZ>::N1 * SZ;
+    constexpr int GX = solve_tb<NX> / Split<NX>::N1 * SX, GZ = solve_tb<NX> / Split<NZ>::N1 * SZ;
     return sizeof(float2) * (size_t)(nz * P + NX + NZ + (GX > GZ ? GX : GZ));
+}
+
+// The field of cell c, column i: the two cubes and, when given, the gather's
+// pairs E4[c] = (Ex, Ez) of columns i and i + 1
+__device__ __forceinline__ void put_field(float *Ex, float *Ez, float4 *E4, int64_t c, int i, float ex, float ez)
+{
+    Ex[c] = ex;
+    Ez[c] = ez;
+    if (!E4) return;
+    float2 *p = reinterpret_cast<float2 *>(E4 + c);
+    p[0] = make_float2(ex, ez);
+    if (i > 0) p[-1] = make_float2(ex, ez);
 }
 
 // One cluster of two blocks per slice (block 2 s + r, r = 0, 1; each pass
@@ -628,9 +711,10 @@ constexpr size_t solve_smem()
 // potential (scaled by 1 / (NX NZ) as the normalised inverse does) and the
 // field cubes; the charge cube as float32 on the way in.
 template <int NX, int NZ, bool HOCK>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SOLVE_TB, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(solve_tb<NX>, 1)
     sc_solve_fused(const unsigned long long *__restrict__ acc, const SCState *st, const float *__restrict__ gk,
-                   float *__restrict__ rho, float *__restrict__ phi, float *__restrict__ Ex, float *__restrict__ Ez)
+                   float *__restrict__ rho, float *__restrict__ phi, float *__restrict__ Ex, float *__restrict__ Ez,
+                   float4 *__restrict__ E4)
 {
     // a cluster of two CTAs per slice: each holds the whole half spectrum,
     // transforms every second line of each pass, and stores its results in
@@ -649,10 +733,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SOLVE_TB, 1)
     float2 *scr = twz + NZ;
     float2 *peer = cluster.map_shared_rank(spec, rank ^ 1);
     const int tid = threadIdx.x;
+    for (int m = tid; m < NX; m += solve_tb<NX>) {
+        double sv, cv;
+        sincospi(2.0 * (double)m / (double)NX, &sv, &cv);
+        twx[m] = make_float2((float)cv, (float)(-sv));
+    }
+    for (int m = tid; m < NZ; m += solve_tb<NX>) {
+        double sv, cv;
+        sincospi(2.0 * (double)m / (double)NZ, &sv, &cv);
+        twz[m] = make_float2((float)cv, (float)(-sv));
+    }
+    chain_wait();
     const int64_t cube0 = (int64_t)(blockIdx.x >> 1) * nz * nx;
     const int degenerate = st->degenerate, bad = st->bad;
     if (bad) {   // the same for both CTAs: neither touches the other's memory
-        for (int e = tid + rank * SOLVE_TB; e < nz * nx; e += 2 * SOLVE_TB) {
+        for (int e = tid + rank * solve_tb<NX>; e < nz * nx; e += 2 * solve_tb<NX>) {
             rho[cube0 + e] = 0.0f;
             phi[cube0 + e] = 0.0f;
             if (!degenerate) { Ex[cube0 + e] = 0.0f; Ez[cube0 + e] = 0.0f; }
@@ -660,23 +755,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SOLVE_TB, 1)
         return;
     }
     const double qd = st->diag.q_density / FIX_SCALE;
-    for (int m = tid; m < NX; m += SOLVE_TB) {
-        double sv, cv;
-        sincospi(2.0 * (double)m / (double)NX, &sv, &cv);
-        twx[m] = make_float2((float)cv, (float)(-sv));
-    }
-    for (int m = tid; m < NZ; m += SOLVE_TB) {
-        double sv, cv;
-        sincospi(2.0 * (double)m / (double)NZ, &sv, &cv);
-        twz[m] = make_float2((float)cv, (float)(-sv));
-    }
     cluster.sync();   // both CTAs running (and twiddles ready) before any store to the partner
 
     // (1) forward row transforms, two real rows per complex line
     {
         const Grp<X1> g;
         float2 *S = scr + g.gid * SX;
-        constexpr int NPAIR = nz / 2, G = SOLVE_TB / X1;
+        constexpr int NPAIR = nz / 2, G = solve_tb<NX> / X1;
         for (int base = 0; base < (NPAIR + 1) / 2; base += G) {
             const int p = 2 * (base + g.line) + rank;
             const bool act = p < NPAIR;
@@ -722,7 +807,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SOLVE_TB, 1)
     {
         const Grp<Z1> g;
         float2 *S = scr + g.gid * SZ;
-        constexpr int G = SOLVE_TB / Z1;
+        constexpr int G = solve_tb<NX> / Z1;
         float dkx = 0.0f, dkz = 0.0f;
         if (!HOCK) {
             dkx = (float)(2.0 * PI / (nx * st->diag.dx));
@@ -781,7 +866,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SOLVE_TB, 1)
     {
         const Grp<X1> g;
         float2 *S = scr + g.gid * SX;
-        constexpr int NPAIR = nz / 2, G = SOLVE_TB / X1;
+        constexpr int NPAIR = nz / 2, G = solve_tb<NX> / X1;
         const float scale = (float)(1.0 / ((double)NX * (double)NZ));
         for (int base = 0; base < (NPAIR + 1) / 2; base += G) {
             const int p = 2 * (base + g.line) + rank;
@@ -837,9 +922,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SOLVE_TB, 1)
         const double ig2 = 1.0 / (gm * gm);
         const double inv2dr = 0.5 / dr, inv2dz = 0.5 / dz;
         const bool zero = (dr == 0.0 || dz == 0.0 || BL == 0);
-        for (int e = tid + rank * SOLVE_TB; e < nz * nx; e += 2 * SOLVE_TB) {
-            if (zero) { Ex[cube0 + e] = 0.0f; Ez[cube0 + e] = 0.0f; continue; }
+        for (int e = tid + rank * solve_tb<NX>; e < nz * nx; e += 2 * solve_tb<NX>) {
             const int j = e / nx, i = e - j * nx;
+            if (zero) { put_field(Ex, Ez, E4, cube0 + e, i, 0.0f, 0.0f); continue; }
 #define PH(jj, ii) reinterpret_cast<const float *>(spec + (jj) * P)[(ii)]
             double ex, ez;
             if (i == 0 || i == nx - 1) {
@@ -858,8 +943,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SOLVE_TB, 1)
                 ez = -(double)__fsub_rn(PH(j + 1, i), PH(j - 1, i)) * inv2dz * ig2;
             }
 #undef PH
-            Ex[cube0 + e] = (float)ex;
-            Ez[cube0 + e] = (float)ez;
+            put_field(Ex, Ez, E4, cube0 + e, i, (float)ex, (float)ez);
         }
     }
 }
@@ -867,33 +951,52 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SOLVE_TB, 1)
 // grids the fused solve is instantiated for: square, 32 / 64 / 128
 bool fused_grid(int nx, int nz) { return nx == nz && (nx == 32 || nx == 64 || nx == 128); }
 
+// A launch that may begin while the kernel before it in the stream still runs
+// (its kernel calls chain_wait).  It hides the 1-2 us between launches: 100003
+// particles, 32 x 64 x 64 cells 52 -> 44 us.
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 template <int NX, int NZ, bool HOCK>
 cudaError_t launch_fused_t(const unsigned long long *acc, const SCState *st, int ns, const float *gk, float *rho,
-                           float *phi, float *ex, float *ez, cudaStream_t s)
+                           float *phi, float *ex, float *ez, float4 *e4, cudaStream_t s)
 {
     constexpr size_t smem = solve_smem<NX, NZ, HOCK>();
     static_assert(smem <= 227 * 1024, "slice does not fit in shared memory");
     const cudaError_t e = cudaFuncSetAttribute(sc_solve_fused<NX, NZ, HOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)smem);
     if (e != cudaSuccess) return e;
-    sc_solve_fused<NX, NZ, HOCK><<<2 * ns, SOLVE_TB, smem, s>>>(acc, st, gk, rho, phi, ex, ez);   // 2-CTA clusters
-    return cudaGetLastError();
+    // 2-CTA clusters
+    return launch_chained(sc_solve_fused<NX, NZ, HOCK>, 2 * ns, solve_tb<NX>, smem, s, acc, st, gk, rho, phi, ex, ez, e4);
 }
 
 cudaError_t launch_fused(int n, bool hockney, const unsigned long long *acc, const SCState *st, int ns,
-                         const float *gk, float *rho, float *phi, float *ex, float *ez, cudaStream_t s)
+                         const float *gk, float *rho, float *phi, float *ex, float *ez, float4 *e4, cudaStream_t s)
 {
     if (!hockney) {
         switch (n) {
-        case 32: return launch_fused_t<32, 32, false>(acc, st, ns, gk, rho, phi, ex, ez, s);
-        case 64: return launch_fused_t<64, 64, false>(acc, st, ns, gk, rho, phi, ex, ez, s);
-        default: return launch_fused_t<128, 128, false>(acc, st, ns, gk, rho, phi, ex, ez, s);
+        case 32: return launch_fused_t<32, 32, false>(acc, st, ns, gk, rho, phi, ex, ez, e4, s);
+        case 64: return launch_fused_t<64, 64, false>(acc, st, ns, gk, rho, phi, ex, ez, e4, s);
+        default: return launch_fused_t<128, 128, false>(acc, st, ns, gk, rho, phi, ex, ez, e4, s);
         }
     }
     switch (n) {
-    case 32: return launch_fused_t<64, 64, true>(acc, st, ns, gk, rho, phi, ex, ez, s);
-    case 64: return launch_fused_t<128, 128, true>(acc, st, ns, gk, rho, phi, ex, ez, s);
-    default: return launch_fused_t<256, 256, true>(acc, st, ns, gk, rho, phi, ex, ez, s);
+    case 32: return launch_fused_t<64, 64, true>(acc, st, ns, gk, rho, phi, ex, ez, e4, s);
+    case 64: return launch_fused_t<128, 128, true>(acc, st, ns, gk, rho, phi, ex, ez, e4, s);
+    default: return launch_fused_t<256, 256, true>(acc, st, ns, gk, rho, phi, ex, ez, e4, s);
     }
 }
 
@@ -1051,7 +1154,7 @@ __global__ void sc_potential(const float2 *work, ffa_sc_desc d, int NZ, int NX, 
 }
 
 // compute_field_from_potential_numba_SBS for every cell
-__global__ void sc_field(const float *phi, ffa_sc_desc d, const SCState *st, float *Ex, float *Ez)
+__global__ void sc_field(const float *phi, ffa_sc_desc d, const SCState *st, float *Ex, float *Ez, float4 *E4)
 {
     if (st->degenerate) return;
     const int nx = d.nx, nz = d.nz;
@@ -1062,10 +1165,10 @@ __global__ void sc_field(const float *phi, ffa_sc_desc d, const SCState *st, flo
     const int64_t tot = (int64_t)d.ns * nz * nx;
     const bool zero = (dr == 0.0 || dz == 0.0 || BL == 0);
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
-        if (zero) { Ex[e] = 0.0f; Ez[e] = 0.0f; continue; }
         const int64_t s = e / ((int64_t)nz * nx);
         const int64_t rem = e - s * nz * nx;
         const int j = (int)(rem / nx), i = (int)(rem - (int64_t)j * nx);
+        if (zero) { put_field(Ex, Ez, E4, e, i, 0.0f, 0.0f); continue; }
         const float *P = phi + s * nz * nx;
 #define PH(jj, ii) P[(int64_t)(jj) * nx + (ii)]
         double ex, ez;
@@ -1085,8 +1188,7 @@ __global__ void sc_field(const float *phi, ffa_sc_desc d, const SCState *st, flo
             ez = -(double)__fsub_rn(PH(j + 1, i), PH(j - 1, i)) * inv2dz * ig2;
         }
 #undef PH
-        Ex[e] = (float)ex;
-        Ez[e] = (float)ez;
+        put_field(Ex, Ez, E4, e, i, (float)ex, (float)ez);
     }
 }
 
@@ -1114,30 +1216,44 @@ cudaError_t fft2d(float2 *data, int nslices, int NZ, int NX, int lognz, int logn
 // Bilinear field at each live particle, projected on the closed-orbit
 // direction; then, when `roll`, the extrapolation endpoints after the update
 // (src/FFAG_track.py:341-400): pre <- the new field for live particles,
-// pp <- the old pre, and the masks likewise.
+// pp <- the old pre, and the masks likewise.  The field at the cell's corners
+// comes from the solve's pairs E4, two 16-byte loads: each line a warp's load
+// touches costs the L1 data pipe a cycle, and eight 4-byte loads touched them
+// four times (without E4 -- the static update's fixed scratch has no room for
+// it -- they still do).  1e6 particles: 36.5 -> 32.2 us, 128 B a particle at 0.6 of
+// the copy bandwidth.
 __global__ void __launch_bounds__(SC_TB) sc_gather_roll(ffa_state_soa S, int64_t n, ffa_sc_desc d, const double *x,
                                                         const double *pr0, const int32_t *slice, const SCState *st,
-                                                        const float *Ex, const float *Ez, int roll, int first)
+                                                        const float *Ex, const float *Ez, const float4 *E4, int roll,
+                                                        int first)
 {
+    chain_wait();
     const int nx = d.nx, nz = d.nz;
     const int degenerate = st->degenerate, bad = st->bad;
-    const double x0 = st->diag.xmin, z0 = st->diag.zmin, dx = st->diag.dx, dz = st->diag.dz;
+    const double x0 = st->diag.xmin, z0 = st->diag.zmin;
+    const Divisor dx(st->diag.dx, st->inv_dx), dz(st->diag.dz, st->inv_dz);
     auto one = [&](int64_t i, int s, double xi, double zi, double p, uint8_t surv) {
         double er = 0.0, ez = 0.0, ef = 0.0;
         bool fresh = false;
         if (!degenerate && s >= 0) {
             if (!bad) {
-                const float *EX = Ex + (int64_t)s * nz * nx, *EZ = Ez + (int64_t)s * nz * nx;
-                const double t = (xi - x0) / dx, u = (zi - z0) / dz;
-                int64_t i0 = (int64_t)floor(t), j0 = (int64_t)floor(u);
+                const double t = dx.quotient(xi - x0), u = dz.quotient(zi - z0);
+                int i0 = (int)floor(t), j0 = (int)floor(u);
                 if (i0 < 0) i0 = 0; else if (i0 > nx - 2) i0 = nx - 2;
                 if (j0 < 0) j0 = 0; else if (j0 > nz - 2) j0 = nz - 2;
                 const double al = t - (double)i0, be = u - (double)j0;
                 const double w00 = (1.0 - al) * (1.0 - be), w10 = al * (1.0 - be), w01 = (1.0 - al) * be, w11 = al * be;
-                const double gr = w00 * EX[j0 * nx + i0] + w10 * EX[j0 * nx + i0 + 1] + w01 * EX[(j0 + 1) * nx + i0] +
-                                  w11 * EX[(j0 + 1) * nx + i0 + 1];
-                const double gz = w00 * EZ[j0 * nx + i0] + w10 * EZ[j0 * nx + i0 + 1] + w01 * EZ[(j0 + 1) * nx + i0] +
-                                  w11 * EZ[(j0 + 1) * nx + i0 + 1];
+                const int64_t c = ((int64_t)s * nz + j0) * nx + i0;
+                float4 lo, hi;                       // (Ex, Ez) at i0, i0 + 1; rows j0, j0 + 1
+                if (E4) {
+                    lo = E4[c];
+                    hi = E4[c + nx];
+                } else {
+                    lo = make_float4(Ex[c], Ez[c], Ex[c + 1], Ez[c + 1]);
+                    hi = make_float4(Ex[c + nx], Ez[c + nx], Ex[c + nx + 1], Ez[c + nx + 1]);
+                }
+                const double gr = w00 * lo.x + w10 * lo.z + w01 * hi.x + w11 * hi.z;
+                const double gz = w00 * lo.y + w10 * lo.w + w01 * hi.y + w11 * hi.w;
                 const double rt = sqrt(1 + p * p);
                 er = gr * (1 / rt);
                 ez = gz;
@@ -1204,13 +1320,10 @@ struct SCBufs {
     SCState *st;
     unsigned long long *acc;
     float *rho, *phi, *ex, *ez;
+    float4 *e4;           // the gather's field pairs, NULL: none (static update)
+    SeoCell *cells;       // closed-orbit tables by cell, NULL: none (static update, or too many cells)
     float2 *work;         // batched-FFT path only
     double *gT;           // open boundary: Green row sums, (NZ/2 + 1) x (NX/2 + 1)
-    double *gG;           // open boundary: weighted Green points, same shape
-    // open boundary with a plan: the Green transform runs on `side`,
-    // concurrently with the deposit (fork after pass1, join before the solve)
-    cudaStream_t side;
-    cudaEvent_t fork, join;
     float *gk;            // open boundary: Green transform quadrant
 };
 
@@ -1221,28 +1334,21 @@ int run_update(const ffa_sc_desc &d, const SCBufs &b, ffa_state_soa *S, int64_t 
     const int NX = d.hockney ? 2 * d.nx : d.nx, NZ = d.hockney ? 2 * d.nz : d.nz;
     const int64_t cube = (int64_t)d.ns * d.nz * d.nx;
     const unsigned ew = 148 * 8;  // elementwise grids
-    FFA_CHECK_CUDA(cudaMemsetAsync(b.acc, 0, sizeof(unsigned long long) * (cube + 1), s));
-    sc_pass1<<<SC_BLOCKS, SC_TB, 0, s>>>(*S, n, d, b.x, b.pr0, b.part, b.acc + cube, b.st, status);
-    if (d.hockney) {
-        const bool par = b.side != nullptr;
-        const cudaStream_t g = par ? b.side : s;
-        if (par) {
-            FFA_CHECK_CUDA(cudaEventRecord(b.fork, s));
-            FFA_CHECK_CUDA(cudaStreamWaitEvent(b.side, b.fork, 0));
-        }
-        const dim3 gg((NX / 2 + 32) / 32, (NZ / 2 + 32) / 32);
-        const int64_t quad = (int64_t)(NZ / 2 + 1) * (NX / 2 + 1);
-        sc_green_points<<<(unsigned)((quad + 255) / 256), 256, 0, g>>>(NZ, NX, b.st, b.gG);
-        sc_green_rows<<<gg, 256, sizeof(double) * NX, g>>>(NZ, NX, b.st, b.gG, b.gT);
-        sc_green_cols<<<gg, 256, sizeof(double) * NZ, g>>>(NZ, NX, b.st, b.gT, b.gk);
-        FFA_CHECK_CUDA(cudaGetLastError());
-        if (par) FFA_CHECK_CUDA(cudaEventRecord(b.join, b.side));
-    }
-    sc_deposit<<<particle_blocks(n), SC_TB, 0, s>>>(*S, n, d, b.x, b.slice, b.cell, b.st, b.acc);
-    FFA_CHECK_CUDA(cudaGetLastError());
-    if (d.hockney && b.side) FFA_CHECK_CUDA(cudaStreamWaitEvent(s, b.join, 0));
+    // the tables are packed anew for every update (they are the caller's): worth
+    // it where the particles outnumber the cells
+    SeoCell *cells = (d.nE - 1) * (d.nfi - 1) <= n ? b.cells : nullptr;
+    sc_prepare<<<ew, SC_TB, 0, s>>>(d, cube + 1, b.acc, cells);
+    FFA_CHECK_CUDA(launch_chained(sc_pass1, SC_BLOCKS, SC_TB, 0, s, *S, n, d, Divisors(d), cells, b.x, b.pr0, b.part,
+                                  b.acc + cube, b.st, status));
+    const int hx = NX / 2, hz = NZ / 2, rows = d.hockney ? hz + 1 : 0;
+    FFA_CHECK_CUDA(launch_chained(sc_deposit, rows + particle_blocks(n), SC_TB,
+                                  d.hockney ? sizeof(double) * (hx + 1 + NX) : 0, s, *S, n, d, b.x, b.slice, b.cell, b.st,
+                                  b.acc, rows, NX, b.gT));
+    if (d.hockney)
+        FFA_CHECK_CUDA(launch_chained(sc_green_cols, hx + 1, GREEN_TB, sizeof(double) * (hz + 1 + NZ), s, NZ, NX, b.st,
+                                      b.gT, b.gk));
     if (fused_grid(d.nx, d.nz)) {
-        FFA_CHECK_CUDA(launch_fused(d.nx, d.hockney != 0, b.acc, b.st, d.ns, b.gk, b.rho, b.phi, b.ex, b.ez, s));
+        FFA_CHECK_CUDA(launch_fused(d.nx, d.hockney != 0, b.acc, b.st, d.ns, b.gk, b.rho, b.phi, b.ex, b.ez, b.e4, s));
     } else {
         const int lx = ilog2(NX), lz = ilog2(NZ);
         sc_convert<<<ew, 256, 0, s>>>(b.acc, d, b.st, b.rho, b.work, NZ, NX);
@@ -1252,11 +1358,10 @@ int run_update(const ffa_sc_desc &d, const SCBufs &b, ffa_state_soa *S, int64_t 
         else sc_mul_periodic<<<ew, 256, 0, s>>>(b.work, d, b.st);
         FFA_CHECK_CUDA(fft2d(b.work, d.ns, NZ, NX, lz, lx, 1, s));
         sc_potential<<<ew, 256, 0, s>>>(b.work, d, NZ, NX, b.st, b.phi);
-        sc_field<<<ew, 256, 0, s>>>(b.phi, d, b.st, b.ex, b.ez);
+        sc_field<<<ew, 256, 0, s>>>(b.phi, d, b.st, b.ex, b.ez, b.e4);
     }
-    sc_gather_roll<<<particle_blocks(n), SC_TB, 0, s>>>(*S, n, d, b.x, b.pr0, b.slice, b.st, b.ex, b.ez,
-                                                        roll ? 1 : 0, first ? 1 : 0);
-    FFA_CHECK_CUDA(cudaGetLastError());
+    FFA_CHECK_CUDA(launch_chained(sc_gather_roll, particle_blocks(n), SC_TB, 0, s, *S, n, d, b.x, b.pr0, b.slice, b.st,
+                                  b.ex, b.ez, b.e4, roll ? 1 : 0, first ? 1 : 0));
     if (diag) FFA_CHECK_CUDA(cudaMemcpyAsync(diag, &b.st->diag, sizeof(ffa_sc_diag), cudaMemcpyDeviceToDevice, s));
     return FFA_OK;
 }
@@ -1294,12 +1399,9 @@ void free_plan(ffa_sc_plan *p)
 {
     if (!p) return;
     void *ptrs[] = {p->b.x, p->b.pr0, p->b.slice, p->b.cell, p->b.part, p->b.st, p->b.acc, p->b.rho, p->b.phi,
-                    p->b.ex, p->b.ez, p->b.work, p->b.gT, p->b.gG, p->b.gk};
+                    p->b.ex, p->b.ez, p->b.e4, p->b.cells, p->b.work, p->b.gT, p->b.gk};
     for (void *q : ptrs)
         if (q) cudaFree(q);
-    if (p->b.fork) cudaEventDestroy(p->b.fork);
-    if (p->b.join) cudaEventDestroy(p->b.join);
-    if (p->b.side) cudaStreamDestroy(p->b.side);
     free(p);
 }
 
@@ -1333,16 +1435,15 @@ int ffa_sc_plan_create(const ffa_sc_desc *desc, void *stream, ffa_sc_plan **out)
               cudaMalloc(&b.rho, sizeof(float) * cube) == cudaSuccess &&
               cudaMalloc(&b.phi, sizeof(float) * cube) == cudaSuccess &&
               cudaMalloc(&b.ex, sizeof(float) * cube) == cudaSuccess &&
-              cudaMalloc(&b.ez, sizeof(float) * cube) == cudaSuccess;
+              cudaMalloc(&b.ez, sizeof(float) * cube) == cudaSuccess &&
+              cudaMalloc(&b.e4, sizeof(float4) * cube) == cudaSuccess;
+    const int64_t ncells = (d.nE - 1) * (d.nfi - 1);
+    if (ok && ncells <= SEO_CELLS_MAX) ok = cudaMalloc(&b.cells, sizeof(SeoCell) * ncells) == cudaSuccess;
     if (ok && !fused_grid(d.nx, d.nz)) ok = cudaMalloc(&b.work, sizeof(float2) * d.ns * (int64_t)NZ * NX) == cudaSuccess;
     if (ok && d.hockney) {
         const int64_t quad = (int64_t)(NZ / 2 + 1) * (NX / 2 + 1);
         ok = cudaMalloc(&b.gT, sizeof(double) * quad) == cudaSuccess &&
-             cudaMalloc(&b.gG, sizeof(double) * quad) == cudaSuccess &&
-             cudaMalloc(&b.gk, sizeof(float) * quad) == cudaSuccess &&
-             cudaStreamCreateWithFlags(&b.side, cudaStreamNonBlocking) == cudaSuccess &&
-             cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming) == cudaSuccess &&
-             cudaEventCreateWithFlags(&b.join, cudaEventDisableTiming) == cudaSuccess;
+             cudaMalloc(&b.gk, sizeof(float) * quad) == cudaSuccess;
     }
     if (!ok) { free_plan(p); return FFA_ERR_NOMEM; }
     if (cudaMemset(b.st, 0, sizeof(SCState)) != cudaSuccess || cudaMemset(b.slice, 0xff, sizeof(int32_t) * n) != cudaSuccess ||
