@@ -44,11 +44,12 @@ class StepClock:
         self.drf = None
         self.acc = None
 
-    def ensure(self, nsteps: int) -> bool:
-        """Makes tables cover steps [0, nsteps).  Returns True if extended."""
+    def ensure(self, nsteps: int, chunk: int = TABLE_CHUNK) -> bool:
+        """Makes tables cover steps [0, nsteps), extended by at least `chunk`
+        steps.  Returns True if extended."""
         if nsteps <= self.n:
             return False
-        new_n = max(nsteps, self.n + TABLE_CHUNK)
+        new_n = max(nsteps, self.n + chunk)
         add = new_n - self.n
         ext = np.empty(add + 1, dtype=np.float64)
         ext[0] = self.t[-1]
@@ -501,9 +502,12 @@ def single_step(mat, t, dt, gp, solver, precision="fp64"):
     n = a.shape[0]
     dev = torch.device("cuda", torch.cuda.current_device())
     b = _EphemeralBunch(a, solver, dev)
+    # one step needs one table entry (a chunk of 65536 took 1.5 ms of the call's
+    # 2.8 for 2000 particles) and no thread order (sorting costs more than a
+    # step's node loads can gain)
     clock = StepClock(t, dt, gp.Emap, solver, dev)
-    clock.ensure(1)
-    pusher = Pusher(b, gp, solver, precision)
+    clock.ensure(1, chunk=1)
+    pusher = Pusher(b, gp, solver, precision, order=None)
     pusher.push(clock, 0, 1, 0)
     out = b.matrix()
     return out
@@ -520,11 +524,9 @@ class _EphemeralBunch:
         self.n = a.shape[0]
         self._a = a
         self.aos = a.to(dev, torch.float64).contiguous() if torch.is_tensor(a) else torch.from_numpy(a).to(dev)
-        f64 = dict(dtype=torch.float64, device=dev)
-        self.cols = {k: torch.empty(self.n, **f64) for k in ("r", "vr", "z", "vz", "fi", "f5", "rf",
-                                                             "esc_r", "esc_z", "esc_fi")}
-        self.cols["inj"] = torch.empty(self.n, dtype=torch.uint8, device=dev)
-        self.cols["surv"] = torch.empty(self.n, dtype=torch.uint8, device=dev)
+        names = ("r", "vr", "z", "vz", "fi", "f5", "rf", "esc_r", "esc_z", "esc_fi")
+        self.cols = dict(zip(names, torch.empty((len(names), self.n), dtype=torch.float64, device=dev)))
+        self.cols.update(zip(("inj", "surv"), torch.empty((2, self.n), dtype=torch.uint8, device=dev)))
         self.status = torch.zeros(_lib.STATUS_WORDS, dtype=torch.int64, device=dev)
         s = _lib.StateSoA()
         for name, _ in _lib.StateSoA._fields_:
