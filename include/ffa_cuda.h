@@ -496,7 +496,7 @@ int ffa_mapgen(const ffa_mapgen_desc *desc, void *stream);
 #define FFA_MLP_HIDDEN 256
 #define FFA_MLP_PARAMS 138192
 #define FFA_MLP_WPACK_BYTES 278528   /* bfloat16 copies of W1..W4 for inference */
-#define FFA_MLP_SPLIT_WORK 1048576    /* floats of split-K partial products in the training work area */
+#define FFA_MLP_SPLIT_WORK 1048576    /* floats of the training work area beside those per sample */
 
 /* One optimiser step (no counterpart in the reference, whose tracker has no
  * learned map): forward, mean-squared error over the first n_fit
@@ -530,8 +530,7 @@ int ffa_mlp_train_step(const ffa_mlp_train_desc *desc, void *stream);
 /* No counterpart in the reference (part of the learned map's training).
  * C[M][N] = op(A) op(B) (+ bias[N]) in bfloat16 x bfloat16 -> float32 on
  * the tensor cores; op(A)[m][k] = A[m lda + k] (transA 0) or A[k lda + m],
- * op(B)[k][n] = B[k ldb + n] (transB 0) or B[n ldb + k].  The training step's
- * building block, exported for tests. */
+ * op(B)[k][n] = B[k ldb + n] (transB 0) or B[n ldb + k]. */
 int ffa_mlp_gemm(const float *A, int lda, int transA, const float *B, int ldb, int transB, float *C, int ldc,
                  int M, int N, int K, const float *bias, void *stream);
 

@@ -2,16 +2,13 @@
 //
 // y = x + x Ws + bs + f(x),  f = L4 . SiLU . L3 . SiLU . L2 . SiLU . L1,
 // widths 6 -> 256 -> 256 -> 256 -> 6.  Weights are float32 masters, rounded to
-// bfloat16 where they enter an MMA; products accumulate in float32
-// (mma.sync m16n8k16 bf16 -> f32).  The skip layer (Ws, bs) stays float32.
+// bfloat16 where they enter an MMA; products accumulate in float32.  The skip layer (Ws, bs) stays float32.
 //
-// Training: a tiled tensor-core GEMM (op(A) op(B) + bias, operands staged in
-// shared memory as bf16 from float32) and element-wise kernels for SiLU, its
-// derivative, the loss gradient, bias gradients and Adam.
-// Inference: one fused kernel per 128 particles that applies the map
-// n_apply times in a row with the state in shared memory and the hidden
-// activations in registers as MMA operand fragments (an accumulator tile of
-// one layer is, lane for lane, an operand tile of the next: no shuffles).
+// Training: one fused kernel per 64 samples runs forward and backward, one more
+// forms the weight gradients, one sums them and takes the Adam step.
+// Inference: one fused kernel per 128 particles applies the map n_apply times
+// in a row.  Both run on tcgen05 with accumulators in tensor memory.  A general
+// product (op(A) op(B) + bias, float32 in and out) is exported beside them.
 #include <cuda_bf16.h>
 
 #include "ffa_internal.cuh"
@@ -35,11 +32,8 @@ constexpr int64_t P_WS = P_B4 + NOUT;             // [NOUT][NOUT] (6 x 6 used)
 constexpr int64_t P_BS = P_WS + NOUT * NOUT;
 constexpr int64_t P_WQ = P_BS + NOUT;             // [16][NOUT] (15 x 6 used)
 constexpr int64_t P_TOTAL = P_WQ + 16 * NOUT;
-// quadratic skip features: s_i s_j for i <= j < 5, in this order
-__device__ __constant__ int8_t QI[15] = {0, 0, 0, 0, 0, 1, 1, 1, 1, 2, 2, 2, 3, 3, 4};
-__device__ __constant__ int8_t QJ[15] = {0, 1, 2, 3, 4, 1, 2, 3, 4, 2, 3, 4, 3, 4, 4};
-
-// the 15 quadratic features of a register-resident state, in QI / QJ order
+// the 15 quadratic skip features s_i s_j, i <= j < 5, of a register-resident
+// state, in the order (0, 0), (0, 1) .. (0, 4), (1, 1) .. (4, 4)
 __device__ __forceinline__ void quad_features(const float *x, float *q)
 {
     q[0] = x[0] * x[0]; q[1] = x[0] * x[1]; q[2] = x[0] * x[2]; q[3] = x[0] * x[3]; q[4] = x[0] * x[4];
@@ -86,7 +80,7 @@ __device__ __forceinline__ float dsilu(float z)
     return 0.5f * (1.0f + t) * fmaf(h, 1.0f - t, 1.0f);
 }
 
-// ------------------------------------------------------------ GEMM (training)
+// ------------------------------------------------------------- GEMM, narrow
 // C[M][N] = op(A)[M][K] op(B)[K][N] (+ bias[N]); op(A)[m][k] = A[m*lda + k]
 // or, with transA, A[k*lda + m]; op(B)[k][n] = B[k*ldb + n] or, with transB,
 // B[n*ldb + k].  64 x 64 block tile, K staged 32 at a time as bf16 in shared
@@ -97,19 +91,12 @@ constexpr int GT_M = 64, GT_N = 64, GT_K = 32, GT_PAD = 8;
 __global__ void __launch_bounds__(128) gemm_tc(const float *__restrict__ A, int lda, int transA,
                                                const float *__restrict__ B, int ldb, int transB,
                                                float *__restrict__ C, int ldc, int M, int N, int K,
-                                               const float *__restrict__ bias, int k_chunk)
+                                               const float *__restrict__ bias)
 {
     __shared__ __align__(16) __nv_bfloat16 sA[GT_M][GT_K + GT_PAD];
     __shared__ __align__(16) __nv_bfloat16 sB[GT_N][GT_K + GT_PAD];
     const int m0 = blockIdx.y * GT_M, n0 = blockIdx.x * GT_N;
-    // split K: block z covers [kb, ke) and writes its partial product to
-    // C + z * M * N (row stride N) when gridDim.z > 1
-    const int kb = blockIdx.z * k_chunk, ke = min(K, kb + k_chunk);
-    if (gridDim.z > 1) {
-        C += (int64_t)blockIdx.z * M * N;
-        ldc = N;
-        bias = nullptr;
-    }
+    const int kb = 0, ke = K;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
     const int r = lane >> 2, c2 = (lane & 3) * 2;
@@ -193,198 +180,8 @@ __global__ void __launch_bounds__(128) gemm_tc(const float *__restrict__ A, int 
             }
 }
 
-// C[m][n] = sum over the splits of part[z][m][n], in split order
-__global__ void split_sum_kernel(const float *__restrict__ part, int splits, int M, int N, float *__restrict__ C,
-                                 int ldc, const float *__restrict__ bias)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M * N) return;
-    float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += part[(int64_t)z * M * N + i];
-    C[(int64_t)(i / N) * ldc + (i % N)] = s + (bias ? bias[i % N] : 0.0f);
-}
+constexpr int64_t SPLIT_WORK = FFA_MLP_SPLIT_WORK;   // floats of the training work area beside those per sample
 
-constexpr int SPLITS_MAX = 16;
-constexpr int64_t SPLIT_WORK = (int64_t)SPLITS_MAX * H * H;   // floats
-static_assert(SPLIT_WORK == FFA_MLP_SPLIT_WORK, "training split-K work area");
-
-// ------------------------------------------------------- element-wise (training)
-// layer 1: z1 = x W1 + b1 with the float32 input and bfloat16-rounded W1, the
-// values the inference kernel's split-input product forms
-__global__ void layer1_kernel(const float *__restrict__ x, const float *__restrict__ P, float *__restrict__ z1,
-                              int64_t B)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < B * H; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / H;
-        const int n = (int)(i - r * H);
-        float z = P[P_B1 + n];
-#pragma unroll
-        for (int k = 0; k < 6; ++k)
-            z = fmaf(x[r * NOUT + k], __bfloat162float(__float2bfloat16_rn(P[P_W1 + k * H + n])), z);
-        z1[i] = z;
-    }
-}
-
-__global__ void silu_kernel(const float *z, float *h, int64_t n)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        h[i] = silu(z[i]);
-}
-
-__global__ void dsilu_kernel(float *dh, const float *z, int64_t n)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dh[i] *= dsilu(z[i]);
-}
-
-// y = x + x Ws + bs + f; d = 2 (y - t) / (B n_fit) on the fitted outputs;
-// per-block partial of the squared error.  x, t: [B][8] float32, f: [B][8].
-__global__ void out_grad_kernel(const float *x, const float *t, const float *f, const float *P, float *y, float *d,
-                                int64_t B, int n_fit, double *loss_part)
-{
-    __shared__ double sh[256];
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < B; i += (int64_t)gridDim.x * blockDim.x) {
-        for (int c = 0; c < NOUT; ++c) {
-            float v = 0.0f;
-            if (c < 6) {
-                v = x[i * NOUT + c] + f[i * NOUT + c] + P[P_BS + c];
-                for (int k = 0; k < 6; ++k) v += x[i * NOUT + k] * P[P_WS + k * NOUT + c];
-                for (int m = 0; m < 15; ++m) v += x[i * NOUT + QI[m]] * x[i * NOUT + QJ[m]] * P[P_WQ + m * NOUT + c];
-            }
-            y[i * NOUT + c] = v;
-            float g = 0.0f;
-            if (c < n_fit) {
-                const float e = v - t[i * NOUT + c];
-                acc += (double)e * (double)e;
-                g = 2.0f * e / (float)(B * n_fit);
-            }
-            d[i * NOUT + c] = g;
-        }
-    }
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) loss_part[blockIdx.x] = sh[0];
-}
-
-// column sums g[c] = sum_i d[i][c]: one block per 32 columns, eight warps
-// over interleaved rows, then a fixed-order reduction (deterministic).
-// Column sums g[c] = sum_i d[i][c] (bias gradients) in two fixed-order
-// passes: block (x, y) sums 32 columns over the rows [y rows_per, (y + 1)
-// rows_per) into part[y][c] (8 warps, 4 rows each per step), then one
-// thread per column adds the partial sums in row-chunk order.
-__global__ void __launch_bounds__(256) colsum_part_kernel(const float *__restrict__ d, int64_t B, int ncol, int ld,
-                                                          int64_t rows_per, float *__restrict__ part)
-{
-    __shared__ float sh[8][33];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int c = blockIdx.x * 32 + lane;
-    const int64_t i0 = blockIdx.y * rows_per, i1 = min(B, i0 + rows_per);
-    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
-    if (c < ncol) {
-        int64_t i = i0 + w;
-        for (; i + 24 < i1; i += 32) {
-            s0 += d[i * ld + c];
-            s1 += d[(i + 8) * ld + c];
-            s2 += d[(i + 16) * ld + c];
-            s3 += d[(i + 24) * ld + c];
-        }
-        for (; i < i1; i += 8) s0 += d[i * ld + c];
-    }
-    sh[w][lane] = (s0 + s1) + (s2 + s3);
-    __syncthreads();
-    if (w == 0 && c < ncol) {
-        float t = 0.0f;
-        for (int k = 0; k < 8; ++k) t += sh[k][lane];
-        part[(int64_t)blockIdx.y * ncol + c] = t;
-    }
-}
-
-// one warp per column: lane l adds chunks l, l + 32, ..., then a fixed
-// shuffle tree (the same order every call)
-__global__ void colsum_final_kernel(const float *__restrict__ part, int chunks, int ncol, float *__restrict__ g)
-{
-    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (c >= ncol) return;
-    float t = 0.0f;
-    for (int y = lane; y < chunks; y += 32) t += part[(int64_t)y * ncol + c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) g[c] = t;
-}
-
-// skip-layer gradients: block k < 8 forms gWs[k][c] = sum_i x[i][k] d[i][c],
-// block 8 + m forms gWq[m][c] = sum_i x[i][QI[m]] x[i][QJ[m]] d[i][c]
-// (c < 6), 256 threads over rows, fixed-order reduction
-__global__ void __launch_bounds__(256) skip_grad_kernel(const float *x, const float *d, int64_t B, float *G)
-{
-    __shared__ float sh[256][NOUT + 1];
-    const int k = blockIdx.x;
-    const bool quad = k >= NOUT;
-    const int m = k - NOUT;
-    float s[NOUT];
-#pragma unroll
-    for (int c = 0; c < NOUT; ++c) s[c] = 0.0f;
-    if ((!quad && k < 6) || (quad && m < 15))
-        for (int64_t i = threadIdx.x; i < B; i += blockDim.x) {
-            const float xk = quad ? x[i * NOUT + QI[m]] * x[i * NOUT + QJ[m]] : x[i * NOUT + k];
-#pragma unroll
-            for (int c = 0; c < 6; ++c) s[c] += xk * d[i * NOUT + c];
-        }
-#pragma unroll
-    for (int c = 0; c < NOUT; ++c) sh[threadIdx.x][c] = s[c];
-    __syncthreads();
-    if (threadIdx.x < NOUT) {
-        float t = 0.0f;
-        for (int i = 0; i < (int)blockDim.x; ++i) t += sh[i][threadIdx.x];
-        G[(quad ? P_WQ + m * NOUT : P_WS + k * NOUT) + threadIdx.x] = t;
-    }
-}
-
-__global__ void adam_kernel(float *P, const float *G, float *m, float *v, int64_t n, float lr, float b1, float b2,
-                            float eps, float c1, float c2, const uint8_t *mask)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        if (mask && !mask[i]) continue;
-        const float g = G[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * g;
-        const float vi = b2 * v[i] + (1.0f - b2) * g * g;
-        m[i] = mi;
-        v[i] = vi;
-        P[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    }
-}
-
-// Adam with the step read from the device: learning rate lr_table[*counter],
-// bias corrections of step *counter + 1
-__global__ void adam_sched_kernel(float *P, const float *G, float *m, float *v, int64_t n, const float *lr_table,
-                                  const int32_t *counter, float b1, float b2, float eps, const uint8_t *mask)
-{
-    const int k = *counter;
-    const float lr = lr_table[k], t = (float)(k + 1);
-    const float c1 = 1.0f - powf(b1, t), c2 = 1.0f - powf(b2, t);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        if (mask && !mask[i]) continue;
-        const float g = G[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * g;
-        const float vi = b2 * v[i] + (1.0f - b2) * g * g;
-        m[i] = mi;
-        v[i] = vi;
-        P[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    }
-}
-
-__global__ void counter_advance_kernel(int32_t *counter) { *counter += 1; }
-
-// ------------------------------------------------------- fused inference
-// 8 warps x 16 particles.  Shared: W2^T as bf16 [n][k + 8] (k padded against
-// bank conflicts), W1^T [n][16], W4^T [8][k + 8], biases, skip layer, the
-// state of the block's 128 particles.  W3^T bf16 [n][k] is read from global
-// (L1 / L2 resident: 128 KB shared by every block).
 // ------------------------------------------------------- fused inference
 // tcgen05 tensor cores, one 128-state tile per CTA at a time (persistent grid,
 // one CTA per SM).  Every layer is one 128 x N accumulator in tensor memory:
@@ -1223,11 +1020,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     if (threadIdx.x == 0 && *abort_flag && error) atomicExch(error, 1);
 }
 
-// ------------------------------------------------- GEMM (training, tcgen05)
-// The training products of at least 128 x 128 x 64 on the 5th-generation
-// tensor cores: C[M][N] = op(A) op(B) (+ bias) with the operands and the
-// meaning of transA / transB of gemm_tc.  One CTA of sixteen warps per
-// 128 x 128 output tile (and per K split, gridDim.z, as in gemm_tc); K is
+// ------------------------------------------------------------ GEMM, tcgen05
+// Products of at least 128 x 128 x 64 on the 5th-generation tensor cores:
+// C[M][N] = op(A) op(B) (+ bias) with the operands and the meaning of transA /
+// transB of gemm_tc.  One CTA of sixteen warps per 128 x 128 output tile; K is
 // staged 64 at a time: every thread loads its 16 + 16 float32 of the step
 // from global memory along the index that is contiguous there (into
 // registers, one step ahead), rounds to bfloat16 (as gemm_tc does) and
@@ -1309,7 +1105,7 @@ __device__ __forceinline__ void g5_store(unsigned char *dst, const float v[G5_PE
 __global__ void __launch_bounds__(G5_THREADS) gemm_tc05(const float *__restrict__ A, int lda, int transA,
                                                         const float *__restrict__ B, int ldb, int transB,
                                                         float *__restrict__ C, int ldc, int M, int N, int K,
-                                                        const float *__restrict__ bias, int k_chunk, int vecA, int vecB)
+                                                        const float *__restrict__ bias, int vecA, int vecB)
 {
     extern __shared__ unsigned char g5_raw[];
     unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(g5_raw) + 1023) & ~uintptr_t(1023));
@@ -1318,12 +1114,7 @@ __global__ void __launch_bounds__(G5_THREADS) gemm_tc05(const float *__restrict_
     volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + G5_SM_MISC + 4);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * G5_BM, n0 = blockIdx.x * G5_BN;
-    const int kb = blockIdx.z * k_chunk, ke = min(K, kb + k_chunk);
-    if (gridDim.z > 1) {
-        C += (int64_t)blockIdx.z * M * N;
-        ldc = N;
-        bias = nullptr;
-    }
+    const int kb = 0, ke = K;
     if (threadIdx.x == 0) {
         for (int s = 0; s < G5_STAGES; ++s) mbar_init(s0 + G5_SM_BAR + 8 * s, 1);
         *abort_flag = 0;
@@ -1426,6 +1217,782 @@ __global__ void __launch_bounds__(G5_THREADS) gemm_tc05(const float *__restrict_
     if (threadIdx.x == 0 && failed) atomicAdd(&g_gemm_timeouts, 1);
 }
 
+// -------------------------------------------------- training step (fused)
+// One optimiser step in four launches (the plain sequence of products and
+// element-wise passes took about 37 and spent its time between them: 254 us for
+// 8192 samples against 5 us of tensor-core work):
+//   train_pack_kernel   W2 / W3 rounded to bfloat16 as B operands, both ways
+//                       round (forward and backward products)
+//   train_tile_kernel   forward and backward of 64 samples per CTA without
+//                       leaving the SM: activations and deltas as bfloat16 A
+//                       operands in shared memory, the pre-activations z2, z3
+//                       and the products in the two 256-column halves of tensor
+//                       memory, z1 formed again from the input where the
+//                       backward pass needs it.  A tile's 64 samples fill the
+//                       128 rows of its products twice: a thread reaches only
+//                       its own rows of tensor memory, so the copy lets eight
+//                       threads instead of four share a sample's epilogues,
+//                       which are the kernel's time (the doubled products
+//                       are not)
+//   train_wgrad_kernel  weight gradients over the batch: the tiles that the
+//                       kernel above left in global memory are MN-major
+//                       operands as they stand (K = the sample), split over
+//                       CTAs
+//   train_update_kernel sums of the splits in a fixed order, Adam
+// The roundings are those of separate products on bfloat16 operands with
+// float32 accumulation: h, delta, x, dd and W rounded where they enter a
+// product, bias sums and the skip layer in float32 from unrounded deltas.
+// 8192 samples: 254 -> 69 us a step (graph replay); the tile kernel is 28 us of it,
+// bound by the latency of its epilogues (5 of them, SiLU and its derivative on
+// 128 columns each way per thread), the products about 6 us.
+constexpr int TT_THREADS = TC_THREADS;                          // weight stream, MMA, 16 epilogue warps
+constexpr int TT_EPI = TT_THREADS - 64;                         // epilogue threads
+constexpr int TS = 64;                                          // samples per tile
+constexpr uint32_t TS_CHUNK = TS * 128;                         // 64 samples x 64 columns, bfloat16
+constexpr int TT_IMG = 4 * (int)TS_CHUNK;                       // a tile in global memory: four swizzled chunks
+constexpr int TT_SMALL = (int)TS_CHUNK;                         // 16 columns in one chunk (x, dd)
+constexpr uint32_t T_A = 0;                                     // two activation buffers, 128 rows
+constexpr uint32_t T_BUF = 4 * A_CHUNK_BYTES;
+constexpr uint32_t T_RING = T_A + 2 * T_BUF;
+constexpr uint32_t T_W1 = T_RING + 2 * W_CHUNK_BYTES;           // float [6][256], rounded to bfloat16
+constexpr uint32_t T_W4 = T_W1 + 6 * H * 4;                     // float [256][8], rounded to bfloat16
+constexpr uint32_t T_BIAS = T_W4 + H * NOUT * 4;                // b1, b2, b3
+constexpr uint32_t T_F = T_BIAS + 3 * H * 4;                    // partial outputs [8][6][64], then skip features [22][64 + 1]
+constexpr uint32_t T_SKIP = T_F + 8 * 6 * TS * 4;               // b4[8] Ws[64] bs[8] Wq[128]
+constexpr uint32_t T_DD = T_SKIP + 208 * 4;                     // output gradients [6][64 + 1]
+constexpr uint32_t T_BAR = T_DD + 6 * (TS + 1) * 4;             // a_ready[2][4], d_full, f_ready, full[2], empty[2], drain
+constexpr uint32_t T_MISC = T_BAR + 15 * 8;
+constexpr size_t TT_SMEM = T_MISC + 16 + 1024;
+static_assert(TT_SMEM <= 232448, "training tile: shared memory per block");
+static_assert(22 * (TS + 1) <= 8 * 6 * TS, "training tile: skip features");
+static_assert(T_BAR % 8 == 0 && T_SKIP % 16 == 0, "training tile: alignment");
+
+constexpr int SKIP_SUMS = 22 * 6;                               // skip-layer sums: x0..x5, the 15 products, 1, times dd
+constexpr int TG_SPLITS = 16, TG_SMALL_SPLITS = 8;
+
+// the step's scratch inside the caller's work area
+struct TrainWork {
+    int64_t T;                  // tiles
+    int S, SS;                  // splits of the large and small weight gradients
+    unsigned char *img;         // h1 h2 h3 dz1 dz2 dz3: [6][T] tiles
+    unsigned char *small;       // x, dd: [2][T] small tiles
+    unsigned char *wpk;         // W2, W3 forward, W2, W3 backward: 4 x 128 KB
+    float *part;                // [2][S] partial gW2, gW3: [n / 4][k][4]
+    float *part16;              // [2][SS] partial gW1, gW4: [16][256]
+    float *bias;                // [3][2 T][256] sums of dz1, dz2, dz3
+    float *skip;                // [T][SKIP_SUMS]
+    double *loss;               // [2 T]
+    int32_t *ticket;
+};
+
+__host__ __device__ inline unsigned char *tile_img(const TrainWork &w, int arr, int64_t t)
+{
+    return w.img + ((int64_t)arr * w.T + t) * TT_IMG;
+}
+
+__global__ void __launch_bounds__(256) train_pack_kernel(const float *__restrict__ P, TrainWork w)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;       // H * H / 4 threads
+    if (t == 0) *w.ticket = 0;
+    const int k = t / (H / 4), n = 4 * (t % (H / 4));
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+        const float *W = P + (l == 0 ? P_W2 : P_W3) + k * H + n;
+        const float v[4] = {W[0], W[1], W[2], W[3]};
+        unsigned char *f = w.wpk + l * 4 * W_CHUNK_BYTES, *b = w.wpk + (2 + l) * 4 * W_CHUNK_BYTES;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<__nv_bfloat16 *>(f + swz_off(n + i, k, H)) = __float2bfloat16_rn(v[i]);
+        *reinterpret_cast<uint2 *>(b + swz_off(k, n, H)) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+    }
+}
+
+__device__ __forceinline__ void bulk_store(void *dst, uint32_t src, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// Sums over the warp's 32 rows of 8 columns: lane l ends with column l & 7.
+// Each of the first three exchanges halves the columns a lane keeps: nine
+// shuffles in all.
+__device__ __forceinline__ float warp_colsum8(float (&v)[8])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int s = 4; s >= 1; s >>= 1) {
+        const bool up = (lane & s) != 0;
+#pragma unroll
+        for (int i = 0; i < s; ++i) {
+            const float mine = up ? v[i + s] : v[i], theirs = up ? v[i] : v[i + s];
+            v[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, s);
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 8);
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+}
+
+__device__ __forceinline__ void tmem_load8(uint32_t addr, float (&v)[8])
+{
+    uint32_t u[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+                 : "r"(addr));
+    tmem_wait_ld();
+    asm volatile("" : "+r"(u[0]), "+r"(u[1]), "+r"(u[2]), "+r"(u[3]), "+r"(u[4]), "+r"(u[5]), "+r"(u[6]), "+r"(u[7]));
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(u[j]);
+}
+
+__device__ __forceinline__ void tmem_load8x2(uint32_t a, uint32_t b, float (&v)[8], float (&y)[8])
+{
+    uint32_t u[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+                 : "r"(a));
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+                 : "r"(b));
+    tmem_wait_ld();
+    REG_FENCE16(u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        v[j] = __uint_as_float(u[j]);
+        y[j] = __uint_as_float(u[8 + j]);
+    }
+}
+
+__device__ __forceinline__ uint4 pack8(const float (&v)[8])
+{
+    return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+}
+
+__device__ __forceinline__ void load8(const float *p, float (&v)[8])       // 16-byte aligned
+{
+    const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+// NO: outputs evaluated, 4 (n_fit <= 4) or 6
+template <int NO>
+__global__ void __launch_bounds__(TT_THREADS, 1)
+    train_tile_kernel(const float *__restrict__ P, const float *__restrict__ X, const float *__restrict__ Y, TrainWork w,
+                      int64_t B, int n_fit)
+{
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t s0 = smem_u32(sm);
+    float *sw1 = reinterpret_cast<float *>(sm + T_W1), *sw4 = reinterpret_cast<float *>(sm + T_W4);
+    float *sbias = reinterpret_cast<float *>(sm + T_BIAS), *sf = reinterpret_cast<float *>(sm + T_F);
+    float *stail = reinterpret_cast<float *>(sm + T_SKIP);      // b4[0..7], Ws[8..71], bs[72..79], Wq[80..207]
+    float *sdd = reinterpret_cast<float *>(sm + T_DD);
+    const uint32_t BAR_A = s0 + T_BAR, BAR_D = BAR_A + 64, BAR_FR = BAR_A + 72, BAR_FULL = BAR_A + 80,
+                   BAR_EMPTY = BAR_A + 96, BAR_DRAIN = BAR_A + 112;
+    uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(sm + T_MISC);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + T_MISC + 4);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int c = 0; c < 8; ++c) mbar_init(BAR_A + 8 * c, 16);
+        mbar_init(BAR_D, 1);
+        mbar_init(BAR_FR, 16);
+        for (int r = 0; r < 2; ++r) {
+            mbar_init(BAR_FULL + 8 * r, 1);
+            mbar_init(BAR_EMPTY + 8 * r, 1);
+        }
+        mbar_init(BAR_DRAIN, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = threadIdx.x; i < 6 * H; i += blockDim.x) sw1[i] = __bfloat162float(__float2bfloat16_rn(P[P_W1 + i]));
+    for (int i = threadIdx.x; i < H * NOUT; i += blockDim.x) sw4[i] = __bfloat162float(__float2bfloat16_rn(P[P_W4 + i]));
+    for (int i = threadIdx.x; i < 3 * H; i += blockDim.x) sbias[i] = P[(i < H ? P_B1 : i < 2 * H ? P_B2 : P_B3) + (i % H)];
+    for (int i = threadIdx.x; i < 208; i += blockDim.x)
+        stail[i] = i < 8 ? P[P_B4 + i] : i < 72 ? P[P_WS + (i - 8)] : i < 80 ? P[P_BS + (i - 72)] : P[P_WQ + (i - 80)];
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)),
+                     "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_before_sync();
+    __syncthreads();
+    tc_after_sync();
+    const uint32_t tmem = *tmem_holder;
+    // products in order: h1 W2 -> D0 (z2), h2 W3 -> D1 (z3), dz3 W3^T -> D1, dz2 W2^T -> D1;
+    // operand buffers: h1 0, h2 1, h3 0, dz3 1, dz2 0, dz1 1
+
+    if (warp == 0) {
+        // ---------------------------------------------------- weight stream
+        if (lane == 0) {
+            const int mat[4] = {0, 1, 3, 2};
+            uint32_t q = 0;
+            ffa::chain_wait();                                  // the packed weights
+            for (int64_t t = blockIdx.x; t < w.T && !*abort_flag; t += gridDim.x)
+                for (int l = 0; l < 4; ++l)
+                    for (int c = 0; c < 4; ++c, ++q) {
+                        const uint32_t slot = q & 1;
+                        if (!mbar_wait(BAR_EMPTY + 8 * slot, ((q >> 1) & 1) ^ 1, abort_flag)) goto stream_end;
+                        mbar_expect_tx(BAR_FULL + 8 * slot, W_CHUNK_BYTES);
+                        bulk_load(s0 + T_RING + slot * W_CHUNK_BYTES, w.wpk + (4 * mat[l] + c) * W_CHUNK_BYTES,
+                                  W_CHUNK_BYTES, BAR_FULL + 8 * slot);
+                    }
+        stream_end:
+            // every issued copy has landed before the block exits
+            for (uint32_t r = q > 2 ? q - 2 : 0; r < q; ++r)
+                if (!mbar_wait_bounded(BAR_FULL + 8 * (r & 1), (r >> 1) & 1)) *abort_flag = 1;
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------- MMA issue, tile stores
+        if (lane == 0) {
+            constexpr uint32_t ID = idesc_bf16(TC_M, H);
+            const int arr[6] = {0, 1, 2, 5, 4, 3};              // h1 h2 h3 dz3 dz2 dz1
+            uint32_t q = 0, na[2] = {0, 0};
+            bool ok = true;
+            for (int64_t t = blockIdx.x; t < w.T && ok; t += gridDim.x)
+                for (int l = 0; l < 6 && ok; ++l) {
+                    // a buffer's barriers: its next writer waits for a d_full
+                    // that is committed after this use, so they are never two
+                    // phases ahead
+                    const uint32_t a0 = s0 + T_A + (l & 1) * T_BUF, bar_a = BAR_A + 32 * (l & 1), ph = na[l & 1]++ & 1;
+                    const bool product = l != 2 && l != 5;
+                    const uint32_t D = tmem + (l == 0 ? 0u : 256u);
+                    // the backward products overwrite the half that the
+                    // epilogue reads up to its last chunk
+                    if (l >= 3)
+                        for (int c = 0; c < 4 && ok; ++c) ok = mbar_wait(bar_a + 8 * c, ph, abort_flag);
+                    for (int c = 0; c < 4 && ok; ++c) {
+                        ok = mbar_wait(bar_a + 8 * c, ph, abort_flag);
+                        if (ok && product) ok = mbar_wait(BAR_FULL + 8 * (q & 1), (q >> 1) & 1, abort_flag);
+                        if (!ok) break;
+                        bulk_store(tile_img(w, arr[l], t) + c * TS_CHUNK, a0 + c * A_CHUNK_BYTES, TS_CHUNK);
+                        if (product) {
+                            tc_after_sync();
+                            const uint32_t ac = a0 + c * A_CHUNK_BYTES, bc = s0 + T_RING + (q & 1) * W_CHUNK_BYTES;
+#pragma unroll
+                            for (int kk = 0; kk < 4; ++kk)
+                                umma(D, sdesc(ac + 32 * kk, 16, 1024, 2), sdesc(bc + 32 * kk, 16, 1024, 2), ID, (c | kk) != 0);
+                            umma_commit(BAR_EMPTY + 8 * (q & 1));
+                            ++q;
+                        }
+                    }
+                    if (!ok) break;
+                    bulk_commit();
+                    // the stores have read a buffer before the d_full that lets
+                    // its next writer go on
+                    bulk_wait_read<0>();
+                    if (product) umma_commit(BAR_D);
+                }
+            umma_commit(BAR_DRAIN);
+            if (!mbar_wait_bounded(BAR_DRAIN, 0)) *abort_flag = 1;
+            bulk_wait_all();
+        }
+    } else {
+        // ---------------------------------------------------- epilogue
+        // this thread: sample `smp` of the tile (row `row` of the products, and
+        // its copy 64 rows on or back), columns 8 u .. 8 u + 7 of each chunk
+        const int quarter = warp & 3, u = 2 * ((warp - 2) >> 2) + (quarter >> 1);
+        const int row = quarter * 32 + lane, smp = row & (TS - 1), group = quarter & 1;
+        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + 8 * u;
+        uint32_t nd = 0, nf = 0;
+        bool ok = true;
+        for (int64_t t = blockIdx.x; t < w.T && ok; t += gridDim.x) {
+            const int64_t p = t * TS + smp;
+            const bool in = p < B;
+            float x[6], tg[NO];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) x[k] = in ? X[p * NOUT + k] : 0.0f;
+#pragma unroll
+            for (int c = 0; c < NO; ++c) tg[c] = in ? Y[p * NOUT + c] : 0.0f;
+            auto z1_of = [&](int c, float (&z)[8]) {            // layer 1: float32 x, bfloat16-rounded W1
+                const int n0 = c * TC_CHUNK + 8 * u;
+                load8(sbias + n0, z);
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    float wk[8];
+                    load8(sw1 + k * H + n0, wk);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) z[j] = fmaf(x[k], wk[j], z[j]);
+                }
+            };
+            auto put = [&](int buf, int c, const float (&v)[8]) {   // both copies of the sample's row
+                const uint4 o = pack8(v);
+                unsigned char *a = sm + T_A + buf * T_BUF + c * A_CHUNK_BYTES + smp * 128 + ((u ^ (smp & 7)) << 4);
+                *reinterpret_cast<uint4 *>(a) = o;
+                *reinterpret_cast<uint4 *>(a + TS * 128) = o;
+                fence_async_smem();
+                tc_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR_A + 32 * buf + 8 * c);
+            };
+            auto wait_d = [&]() {
+                ok = __all_sync(0xffffffffu, mbar_wait(BAR_D, nd++ & 1, abort_flag));
+                if (ok) tc_after_sync();
+                return ok;
+            };
+            auto bias_sum = [&](int l, int c, float (&v)[8]) {  // column sums of dz_(l + 1)
+                const float s = warp_colsum8(v);
+                if (lane < 8) w.bias[((int64_t)l * 2 * w.T + 2 * t + group) * H + c * TC_CHUNK + 8 * u + lane] = s;
+            };
+            float z[8], bz[8];
+            // h1 -> buffer 0
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                z1_of(c, z);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) z[j] = silu(z[j]);
+                put(0, c, z);
+            }
+            // h2 -> buffer 1
+            if (!wait_d()) break;
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                tmem_load8(lane_base + c * TC_CHUNK, z);
+                load8(sbias + H + c * TC_CHUNK + 8 * u, bz);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) z[j] = silu(z[j] + bz[j]);
+                put(1, c, z);
+            }
+            // h3 -> buffer 0 (stored only), and this thread's share of h3 W4
+            if (!wait_d()) break;
+            float f[NO];
+#pragma unroll
+            for (int c = 0; c < NO; ++c) f[c] = 0.0f;
+            auto w4_row = [&](int n, float (&v)[NO]) {
+                const float4 wa = *reinterpret_cast<const float4 *>(sw4 + n * NOUT);
+                v[0] = wa.x; v[1] = wa.y; v[2] = wa.z; v[3] = wa.w;
+                if constexpr (NO > 4) {
+                    const float2 wb = *reinterpret_cast<const float2 *>(sw4 + n * NOUT + 4);
+                    v[4] = wb.x; v[5] = wb.y;
+                }
+            };
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                tmem_load8(lane_base + 256 + c * TC_CHUNK, z);
+                load8(sbias + 2 * H + c * TC_CHUNK + 8 * u, bz);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    z[j] = silu(z[j] + bz[j]);
+                    const float hb = __bfloat162float(__float2bfloat16_rn(z[j]));
+                    float wv[NO];
+                    w4_row(c * TC_CHUNK + 8 * u + j, wv);
+#pragma unroll
+                    for (int o = 0; o < NO; ++o) f[o] = fmaf(hb, wv[o], f[o]);
+                }
+                put(0, c, z);
+            }
+#pragma unroll
+            for (int c = 0; c < NO; ++c) sf[(u * 6 + c) * TS + smp] = f[c];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR_FR);
+            ok = __all_sync(0xffffffffu, mbar_wait(BAR_FR, nf++ & 1, abort_flag));
+            if (!ok) break;
+            // outputs, loss and its gradient (every thread of a sample alike)
+            float dd[NO], q[15];
+            quad_features(x, q);
+            double loss = 0.0;
+#pragma unroll
+            for (int c = 0; c < NO; ++c) {
+                float fc = 0.0f;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) fc += sf[(g * 6 + c) * TS + smp];
+                float v = x[c] + (fc + stail[c]) + stail[72 + c];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) v += x[k] * stail[8 + k * NOUT + c];
+#pragma unroll
+                for (int m = 0; m < 15; ++m) v += q[m] * stail[80 + m * NOUT + c];
+                dd[c] = 0.0f;
+                if (in && c < n_fit) {
+                    const float e = v - tg[c];
+                    loss += (double)e * (double)e;
+                    dd[c] = 2.0f * e / (float)(B * n_fit);
+                }
+            }
+            if (u == 0) {
+                // x and dd as operands of the weight gradients, 16 columns
+                unsigned char *sx = w.small + t * TT_SMALL + smp * 128, *sd = w.small + (w.T + t) * TT_SMALL + smp * 128;
+                const float xv[8] = {x[0], x[1], x[2], x[3], x[4], x[5]};
+                float dv[8] = {};
+#pragma unroll
+                for (int c = 0; c < NO; ++c) dv[c] = dd[c];
+                const int s7 = smp & 7;
+                *reinterpret_cast<uint4 *>(sx + ((0 ^ s7) << 4)) = pack8(xv);
+                *reinterpret_cast<uint4 *>(sx + ((1 ^ s7) << 4)) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4 *>(sd + ((0 ^ s7) << 4)) = pack8(dv);
+                *reinterpret_cast<uint4 *>(sd + ((1 ^ s7) << 4)) = make_uint4(0, 0, 0, 0);
+            } else if (u == 2) {
+                for (int off = 16; off > 0; off >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, off);
+                if (lane == 0) w.loss[2 * t + group] = loss;
+            } else if (u == 4) {
+#pragma unroll
+                for (int c = 0; c < 6; ++c) sdd[c * (TS + 1) + smp] = c < NO ? dd[c < NO ? c : 0] : 0.0f;
+            }
+#pragma unroll
+            for (int c = 0; c < NO; ++c) dd[c] = __bfloat162float(__float2bfloat16_rn(dd[c]));
+            // dz3 = (dd W4^T) SiLU'(z3) -> buffer 1
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                tmem_load8(lane_base + 256 + c * TC_CHUNK, z);
+                load8(sbias + 2 * H + c * TC_CHUNK + 8 * u, bz);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    float wv[NO];
+                    w4_row(c * TC_CHUNK + 8 * u + j, wv);
+                    float dh = dd[0] * wv[0];
+#pragma unroll
+                    for (int o = 1; o < NO; ++o) dh = fmaf(dd[o], wv[o], dh);
+                    z[j] = dh * dsilu(z[j] + bz[j]);
+                }
+                put(1, c, z);
+                bias_sum(2, c, z);
+            }
+            // dz2 = (dz3 W3^T) SiLU'(z2) -> buffer 0
+            if (!wait_d()) break;
+            // (every warp has read the partial outputs: their place takes the
+            // skip layer's features)
+            if (u == 6) {
+                float q[15];
+                quad_features(x, q);
+#pragma unroll
+                for (int k = 0; k < 6; ++k) sf[k * (TS + 1) + smp] = x[k];
+#pragma unroll
+                for (int k = 0; k < 15; ++k) sf[(6 + k) * (TS + 1) + smp] = q[k];
+                sf[21 * (TS + 1) + smp] = 1.0f;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR_FR);
+            float dh[8];
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                tmem_load8x2(lane_base + c * TC_CHUNK, lane_base + 256 + c * TC_CHUNK, z, dh);
+                load8(sbias + H + c * TC_CHUNK + 8 * u, bz);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) dh[j] *= dsilu(z[j] + bz[j]);
+                put(0, c, dh);
+                bias_sum(1, c, dh);
+            }
+            // dz1 = (dz2 W2^T) SiLU'(z1) -> buffer 1 (stored only)
+            if (!wait_d()) break;
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                tmem_load8(lane_base + 256 + c * TC_CHUNK, dh);
+                z1_of(c, z);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) dh[j] *= dsilu(z[j]);
+                put(1, c, dh);
+                bias_sum(0, c, dh);
+            }
+            // skip-layer sums: four threads a sum, 16 samples each
+            ok = __all_sync(0xffffffffu, mbar_wait(BAR_FR, nf++ & 1, abort_flag));
+            if (!ok) break;
+            const int et = threadIdx.x - 64;
+            for (int e0 = 0; e0 < SKIP_SUMS; e0 += TT_EPI / 4) {
+                const int e = min(e0 + (et >> 2), SKIP_SUMS - 1);
+                const float *fx = sf + (e / 6) * (TS + 1) + 16 * (et & 3), *fd = sdd + (e % 6) * (TS + 1) + 16 * (et & 3);
+                float s = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) s = fmaf(fx[i], fd[i], s);
+                s += __shfl_xor_sync(0xffffffffu, s, 1);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);
+                if ((et & 3) == 0 && e0 + (et >> 2) < SKIP_SUMS) w.skip[t * SKIP_SUMS + e] = s;
+            }
+        }
+        if (!ok && u == 2 && lane == 0)                        // gave up: the loss says so
+            for (int64_t t = blockIdx.x; t < w.T; t += gridDim.x) w.loss[2 * t + group] = __longlong_as_double(0x7FF8000000000000ll);
+    }
+    tc_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        tc_after_sync();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+    }
+    if (threadIdx.x == 0 && *abort_flag) atomicAdd(&g_gemm_timeouts, 1);
+}
+
+// Weight gradients.  Blocks 0 .. 8 S - 1: (product, quadrant, split): 128 x 128
+// of gW2 = h1^T dz2 or gW3 = h2^T dz3 over the split's tiles; the next 2 SS
+// blocks: (dz1^T x, h3^T dd: 256 x 16, two accumulators).  Each tile
+// (K = 64 samples) is a stage of bulk copies, four stages; operands are MN-major: 64 columns of a row
+// contiguous (128 B, swizzled), 8 rows per 1024 B (SBO), the next 64 columns one
+// chunk on (LBO).
+constexpr int TG_THREADS = 128, TG_STAGES = 4;
+constexpr uint32_t TG_STAGE = 5 * TS_CHUNK;                     // 2 + 2 chunks, or 4 + 1
+constexpr uint32_t TG_BAR = TG_STAGES * TG_STAGE;               // full[], empty[]
+constexpr uint32_t TG_MISC = TG_BAR + 16 * TG_STAGES;
+constexpr size_t TG_SMEM = TG_MISC + 16 + 1024;
+
+__global__ void __launch_bounds__(TG_THREADS, 1) train_wgrad_kernel(TrainWork w)
+{
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t s0 = smem_u32(sm), FULL = s0 + TG_BAR, EMPTY = FULL + 8 * TG_STAGES;
+    uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(sm + TG_MISC);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + TG_MISC + 4);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool large = (int)blockIdx.x < 8 * w.S;
+    const int id = large ? blockIdx.x : blockIdx.x - 8 * w.S;
+    const int prod = large ? (id >> 2) & 1 : id & 1, kh = id & 1, nh = (id >> 1) & 1;
+    const int split = large ? id >> 3 : id >> 1, splits = large ? w.S : w.SS;
+    const int64_t t0 = w.T * split / splits, t1 = w.T * (split + 1) / splits;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2 * TG_STAGES; ++i) mbar_init(FULL + 8 * i, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)),
+                     "r"(128));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_before_sync();
+    __syncthreads();
+    tc_after_sync();
+    const uint32_t tmem = *tmem_holder;
+    ffa::chain_wait();
+    if (threadIdx.x == 0) {
+        auto fill = [&](int64_t t, uint32_t q) {                // use q of the ring: tile t
+            const uint32_t sl = q % TG_STAGES, st = s0 + sl * TG_STAGE, bar = FULL + 8 * sl;
+            if (!mbar_wait(EMPTY + 8 * sl, ((q / TG_STAGES) & 1) ^ 1, abort_flag)) return false;
+            if (large) {
+                mbar_expect_tx(bar, 4 * TS_CHUNK);
+                bulk_load(st, tile_img(w, prod, t) + 2 * kh * TS_CHUNK, 2 * TS_CHUNK, bar);
+                bulk_load(st + 2 * TS_CHUNK, tile_img(w, 4 + prod, t) + 2 * nh * TS_CHUNK, 2 * TS_CHUNK, bar);
+            } else {
+                mbar_expect_tx(bar, 5 * TS_CHUNK);
+                bulk_load(st, tile_img(w, prod == 0 ? 3 : 2, t), 4 * TS_CHUNK, bar);
+                bulk_load(st + 4 * TS_CHUNK, w.small + (prod * w.T + t) * TT_SMALL, TS_CHUNK, bar);
+            }
+            return true;
+        };
+        constexpr uint32_t MN = (1u << 15) | (1u << 16);        // both operands MN-major
+        constexpr uint32_t ID_L = idesc_bf16(TC_M, 128) | MN, ID_S = idesc_bf16(TC_M, 16) | MN;
+        uint32_t filled = 0, used = 0;
+        bool ok = true;
+        for (int64_t t = t0; t < t1 && ok; ++t) {
+            while (ok && filled < used + TG_STAGES && t0 + filled < t1) {
+                ok = fill(t0 + filled, filled);
+                if (ok) ++filled;
+            }
+            if (!ok) break;
+            const uint32_t sl = used % TG_STAGES, st = s0 + sl * TG_STAGE;
+            ok = mbar_wait(FULL + 8 * sl, (used / TG_STAGES) & 1, abort_flag);
+            if (!ok) break;
+            tc_after_sync();
+#pragma unroll
+            for (int kk = 0; kk < TS / 16; ++kk) {              // 16 samples a product
+                const uint32_t off = 2048 * kk, acc = t > t0 || kk > 0;
+                if (large) {
+                    umma(tmem, sdesc(st + off, TS_CHUNK, 1024, 2), sdesc(st + 2 * TS_CHUNK + off, TS_CHUNK, 1024, 2), ID_L,
+                         acc);
+                } else {
+                    const uint64_t b = sdesc(st + 4 * TS_CHUNK + off, TS_CHUNK, 1024, 2);
+                    umma(tmem, sdesc(st + off, TS_CHUNK, 1024, 2), b, ID_S, acc);
+                    umma(tmem + 16, sdesc(st + 2 * TS_CHUNK + off, TS_CHUNK, 1024, 2), b, ID_S, acc);
+                }
+            }
+            umma_commit(EMPTY + 8 * sl);
+            ++used;
+        }
+        // every copy has landed and every product is complete
+        for (uint32_t r = used; r < filled; ++r)
+            if (!mbar_wait_bounded(FULL + 8 * (r % TG_STAGES), (r / TG_STAGES) & 1)) *abort_flag = 1;
+        if (used > 0 && !mbar_wait_bounded(EMPTY + 8 * ((used - 1) % TG_STAGES), ((used - 1) / TG_STAGES) & 1)) *abort_flag = 1;
+    }
+    __syncthreads();
+    tc_after_sync();
+    const bool failed = *abort_flag != 0;
+    const int row = 32 * warp + lane;                           // accumulator row
+    const uint32_t base = tmem + ((uint32_t)(32 * warp) << 16);
+    if (large) {
+        float4 *out = reinterpret_cast<float4 *>(w.part) + ((int64_t)prod * w.S + split) * (H * H / 4) +
+                      (int64_t)(32 * nh) * H + 128 * kh + row;
+#pragma unroll 1
+        for (int n = 0; n < 128; n += 32) {
+            uint32_t v[32];
+            TMEM_LD32(base + n, v);
+            tmem_wait_ld();
+            REG_FENCE32(v);
+            if (failed)
+                for (int j = 0; j < 32; ++j) v[j] = 0x7FC00000u;
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+                out[(int64_t)((n + j) / 4) * H] = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
+                                                              __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+        }
+    } else {
+        uint32_t v[32];                                         // 16 columns of rows `row` and 128 + row
+        TMEM_LD32(base, v);
+        tmem_wait_ld();
+        REG_FENCE32(v);
+        float *out = w.part16 + ((int64_t)prod * w.SS + split) * (16 * H);
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            out[(j & 15) * H + 128 * (j >> 4) + row] = __uint_as_float(failed ? 0x7FC00000u : v[j]);
+    }
+    tc_before_sync();
+    __syncthreads();
+    if (warp == 0) {
+        tc_after_sync();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128));
+    }
+    if (threadIdx.x == 0 && failed) atomicAdd(&g_gemm_timeouts, 1);
+}
+
+struct AdamArgs {
+    float *P, *G, *m, *v;
+    const uint8_t *mask;
+    float lr, b1, b2, eps, c1, c2;
+    const float *lr_table;      // device schedule, or NULL
+    int32_t *counter;
+    int update;
+};
+
+__device__ __forceinline__ void adam_one(const AdamArgs &a, int i, float g, float lr, float c1, float c2)
+{
+    a.G[i] = g;
+    if (!a.update || (a.mask && !a.mask[i])) return;
+    const float mi = a.b1 * a.m[i] + (1.0f - a.b1) * g;
+    const float vi = a.b2 * a.v[i] + (1.0f - a.b2) * g * g;
+    a.m[i] = mi;
+    a.v[i] = vi;
+    a.P[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + a.eps);
+}
+
+// Every parameter's gradient from the partial sums, in a fixed order, then Adam.
+// Blocks 0 .. 255: 32 k x 16 n of W2 and W3 (summed along k, which is contiguous
+// in the partial products, updated along n); then 32 parameters a block, the
+// partial sums of each over eight warps; the loss in the last block.
+constexpr int TU_TILES = 2 * (H / 32) * (H / 16);
+constexpr int TU_REST = (int)(P_TOTAL - 2 * H * H), TU_BLOCKS = TU_TILES + (TU_REST + 31) / 32 + 1;
+
+__global__ void __launch_bounds__(256) train_update_kernel(TrainWork w, AdamArgs a, double *__restrict__ loss_part)
+{
+    __shared__ float sh[32][33];
+    ffa::chain_wait();
+    float lr = a.lr, c1 = a.c1, c2 = a.c2;
+    if (a.lr_table) {
+        const int k = *a.counter;
+        const float t = (float)(k + 1);
+        lr = a.lr_table[k];
+        c1 = 1.0f - powf(a.b1, t);
+        c2 = 1.0f - powf(a.b2, t);
+    }
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    if ((int)blockIdx.x < TU_TILES) {
+        const int prod = blockIdx.x / (TU_TILES / 2), tile = blockIdx.x % (TU_TILES / 2);
+        const int k0 = 32 * (tile / (H / 16)), n0 = 16 * (tile % (H / 16));
+        // warp wp: columns n0 + 4 (wp & 3) .., the splits of one parity
+        const float4 *src = reinterpret_cast<const float4 *>(w.part) + (int64_t)prod * w.S * (H * H / 4) +
+                            (int64_t)(n0 / 4 + (wp & 3)) * H + k0 + lane;
+        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 8
+        for (int z = wp >> 2; z < w.S; z += 2) {
+            const float4 v = __ldg(src + (int64_t)z * (H * H / 4));
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        float *d = &sh[lane][16 * (wp >> 2) + 4 * (wp & 3)];
+        d[0] = s.x; d[1] = s.y; d[2] = s.z; d[3] = s.w;
+        __syncthreads();
+        const int base = (int)(prod == 0 ? P_W2 : P_W3), n = tid & 15;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int k = (tid >> 4) + 16 * j;
+            adam_one(a, base + (k0 + k) * H + n0 + n, sh[k][n] + sh[k][16 + n], lr, c1, c2);
+        }
+    } else if (blockIdx.x + 1 < gridDim.x) {
+        // parameter r of W1, b1, b2, b3, W4, b4, Ws, bs, Wq: its partial sums
+        // lie `ld` apart, `cnt` of them, from `p` (none: the gradient is 0)
+        const int r = (blockIdx.x - TU_TILES) * 32 + lane;
+        const int L1 = KIN * H, L4 = H * NOUT;
+        int i = -1;
+        const float *p = nullptr;
+        int64_t cnt = 0, ld = 0;
+        auto small = [&](int prod, int c, int n) {
+            p = w.part16 + (int64_t)prod * w.SS * (16 * H) + c * H + n;
+            cnt = w.SS;
+            ld = 16 * H;
+        };
+        auto skip = [&](int m, int c) {
+            if (m >= 22 || c >= 6) return;
+            p = w.skip + 6 * m + c;
+            cnt = w.T;
+            ld = SKIP_SUMS;
+        };
+        if (r < L1) {
+            i = (int)P_W1 + r;
+            if (r / H < 6) small(0, r / H, r % H);
+        } else if (r < L1 + 3 * H) {
+            const int l = (r - L1) / H, n = (r - L1) % H;
+            i = (int)(l == 0 ? P_B1 : l == 1 ? P_B2 : P_B3) + n;
+            p = w.bias + (int64_t)l * 2 * w.T * H + n;
+            cnt = 2 * w.T;
+            ld = H;
+        } else if (r < L1 + 3 * H + L4) {
+            const int e = r - L1 - 3 * H;
+            i = (int)P_W4 + e;
+            small(1, e % NOUT, e / NOUT);
+        } else if (r < TU_REST) {
+            const int e = r - L1 - 3 * H - L4, m = e / NOUT;    // b4, Ws (8), bs, Wq (16)
+            i = (int)P_B4 + e;
+            if (m == 0 || m == 9) skip(21, e % NOUT);
+            else if (m < 9) { if (m - 1 < 6) skip(m - 1, e % NOUT); }
+            else if (m - 10 < 15) skip(6 + m - 10, e % NOUT);
+        }
+        float s = 0.0f;
+#pragma unroll 8
+        for (int64_t z = wp; z < cnt; z += 8) s += __ldg(p + z * ld);
+        sh[wp][lane] = s;
+        __syncthreads();
+        if (wp == 0 && i >= 0) {
+            float g = 0.0f;
+            for (int k = 0; k < 8; ++k) g += sh[k][lane];
+            adam_one(a, i, g, lr, c1, c2);
+        }
+    } else {
+        for (int q = tid; q < 148; q += 256) {
+            double s = 0.0;
+            for (int64_t z = q; z < 2 * w.T; z += 148) s += w.loss[z];
+            loss_part[q] = s;
+        }
+    }
+    // the last block to finish advances the schedule
+    if (a.counter) {
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            if (atomicAdd(w.ticket, 1) == (int)gridDim.x - 1) *a.counter += 1;
+        }
+    }
+}
+
+// Places the scratch in the caller's work area; false if it does not fit
+// (it always does: 8 * 256 + 24 floats a sample and SPLIT_WORK are more)
+bool train_layout(TrainWork &w, float *work, int64_t B)
+{
+    w.T = (B + TS - 1) / TS;
+    w.S = (int)((w.T + 1) / 2 < TG_SPLITS ? (w.T + 1) / 2 : TG_SPLITS);      // at least two tiles each
+    w.SS = (int)(w.T < TG_SMALL_SPLITS ? w.T : TG_SMALL_SPLITS);
+    unsigned char *p = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(work) + 127) & ~uintptr_t(127));
+    auto take = [&](int64_t bytes) {
+        unsigned char *q = p;
+        p += (bytes + 127) & ~int64_t(127);
+        return q;
+    };
+    w.img = take(6 * w.T * TT_IMG);
+    w.small = take(2 * w.T * TT_SMALL);
+    w.wpk = take(16 * (int64_t)W_CHUNK_BYTES);
+    w.part = reinterpret_cast<float *>(take(2 * (int64_t)w.S * H * H * 4));
+    w.part16 = reinterpret_cast<float *>(take(2 * (int64_t)w.SS * 16 * H * 4));
+    w.bias = reinterpret_cast<float *>(take(3 * 2 * w.T * H * 4));
+    w.skip = reinterpret_cast<float *>(take(w.T * SKIP_SUMS * 4));
+    w.loss = reinterpret_cast<double *>(take(2 * w.T * 8));
+    w.ticket = reinterpret_cast<int32_t *>(take(4));
+    const int64_t have = (8 * B * H + 24 * B + SPLIT_WORK) * 4;
+    return p - reinterpret_cast<unsigned char *>(work) <= have;
+}
+
 bool g5_fits(int M, int N, int K) { return M >= G5_BM && N >= G5_BN && K >= G5_BK; }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -1433,29 +2000,20 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 // one GEMM launch: the tcgen05 kernel for products of at least one full
 // tile, gemm_tc for the narrow ones (N = 8 outputs, K = 8 inputs, M = 6)
 cudaError_t launch_gemm(const float *A, int lda, int tA, const float *B, int ldb, int tB, float *C, int ldc, int M,
-                        int N, int K, const float *bias, int k_chunk, int splits, cudaStream_t s)
+                        int N, int K, const float *bias, cudaStream_t s)
 {
     if (g5_fits(M, N, K)) {
-        // once per process (one process per GPU); set outside any graph
-        // capture: the first training step runs directly before the capture
-        static bool attr = false;
-        if (!attr) {
-            const cudaError_t e = cudaFuncSetAttribute(gemm_tc05, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)G5_SMEM);
-            if (e != cudaSuccess) return e;
-            attr = true;
-        }
-        const dim3 grid((unsigned)((N + G5_BN - 1) / G5_BN), (unsigned)((M + G5_BM - 1) / G5_BM), (unsigned)splits);
+        const cudaError_t e = cudaFuncSetAttribute(gemm_tc05, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G5_SMEM);
+        if (e != cudaSuccess) return e;
+        const dim3 grid((unsigned)((N + G5_BN - 1) / G5_BN), (unsigned)((M + G5_BM - 1) / G5_BM));
         const int vA = !tA && (lda & 3) == 0 && aligned16(A), vB = tB && (ldb & 3) == 0 && aligned16(B);
-        gemm_tc05<<<grid, G5_THREADS, G5_SMEM, s>>>(A, lda, tA, B, ldb, tB, C, ldc, M, N, K, bias, k_chunk, vA, vB);
+        gemm_tc05<<<grid, G5_THREADS, G5_SMEM, s>>>(A, lda, tA, B, ldb, tB, C, ldc, M, N, K, bias, vA, vB);
     } else {
-        const dim3 grid((unsigned)((N + GT_N - 1) / GT_N), (unsigned)((M + GT_M - 1) / GT_M), (unsigned)splits);
-        gemm_tc<<<grid, 128, 0, s>>>(A, lda, tA, B, ldb, tB, C, ldc, M, N, K, bias, k_chunk);
+        const dim3 grid((unsigned)((N + GT_N - 1) / GT_N), (unsigned)((M + GT_M - 1) / GT_M));
+        gemm_tc<<<grid, 128, 0, s>>>(A, lda, tA, B, ldb, tB, C, ldc, M, N, K, bias);
     }
     return cudaGetLastError();
 }
-
-int blocks_for(int64_t n, int tb) { return (int)((n + tb - 1) / tb < 4096 ? (n + tb - 1) / tb : 4096); }
 
 }  // namespace
 
@@ -1471,7 +2029,7 @@ extern "C" int ffa_mlp_gemm(const float *A, int lda, int transA, const float *B,
 {
     if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return FFA_ERR_INVALID;
     if ((M + GT_M - 1) / GT_M > 65535) return FFA_ERR_UNSUPPORTED;
-    return launch_gemm(A, lda, transA ? 1 : 0, B, ldb, transB ? 1 : 0, C, ldc, M, N, K, bias, K, 1,
+    return launch_gemm(A, lda, transA ? 1 : 0, B, ldb, transB ? 1 : 0, C, ldc, M, N, K, bias,
                        (cudaStream_t)stream) == cudaSuccess ? FFA_OK : FFA_ERR_CUDA;
 }
 
@@ -1497,102 +2055,25 @@ extern "C" int ffa_mlp_train_step(const ffa_mlp_train_desc *d, void *stream)
     cudaStream_t s = (cudaStream_t)stream;
     const int64_t B = d->batch;
     if (B > 65535LL * GT_M || B * H > INT32_MAX) return FFA_ERR_UNSUPPORTED;
-    float *P = d->params, *G = d->grads;
-    float *z1 = d->work, *h1 = z1 + B * H, *z2 = h1 + B * H, *h2 = z2 + B * H, *z3 = h2 + B * H, *h3 = z3 + B * H;
-    float *f = h3 + B * H, *y = f + B * NOUT, *dd = y + B * NOUT, *dh = dd + B * NOUT, *dz = dh + B * H;
-    const int ew = blocks_for(B * H, 256);
-    const int Bi = (int)B;
-    float *part = dz + B * H;                                    // split-K partials
-    // split K over `splits` blocks per output tile (chunks a multiple of
-    // `kq`), partials in the split-K area, summed in a fixed order (+ bias)
-    auto gemm_split = [&](const float *A_, int lda_, int tA_, const float *B_, int ldb_, int tB_, float *C_, int ldc_,
-                          int M_, int N_, int K_, const float *bias_, int splits, int kq) {
-        const int kc = ((K_ + splits - 1) / splits + kq - 1) / kq * kq;
-        splits = (K_ + kc - 1) / kc;
-        if (splits <= 1) {
-            launch_gemm(A_, lda_, tA_, B_, ldb_, tB_, C_, ldc_, M_, N_, K_, bias_, K_, 1, s);
-        } else {
-            launch_gemm(A_, lda_, tA_, B_, ldb_, tB_, part, N_, M_, N_, K_, nullptr, kc, splits, s);
-            split_sum_kernel<<<(M_ * N_ + 255) / 256, 256, 0, s>>>(part, splits, M_, N_, C_, ldc_, bias_);
-        }
-    };
-    auto max_splits = [&](int M_, int N_, int cap) {
-        const int64_t room = SPLIT_WORK / ((int64_t)M_ * N_);
-        return (int)(room < cap ? room : cap);
-    };
-    // products: the tcgen05 kernel whole; the narrow ones (N = 8 outputs)
-    // split in K chunks of 64, as the partial-product area allows
-    auto gemm = [&](const float *A_, int lda_, int tA_, const float *B_, int ldb_, int tB_, float *C_, int ldc_,
-                    int M_, int N_, int K_, const float *bias_) {
-        int splits = 1;
-        if (!g5_fits(M_, N_, K_) && K_ >= 128) {
-            splits = (K_ + 63) / 64;
-            const int cap = max_splits(M_, N_, 64);
-            splits = splits < cap ? splits : cap;
-        }
-        gemm_split(A_, lda_, tA_, B_, ldb_, tB_, C_, ldc_, M_, N_, K_, bias_, splits < 1 ? 1 : splits, GT_K);
-    };
-    // weight gradients (K = batch): chunks of 512 on the tcgen05 path (up to
-    // 16 splits), 256 on gemm_tc (up to 64)
-    auto gemm_wgrad = [&](const float *A_, int lda_, const float *B_, int ldb_, float *C_, int ldc_, int M_, int N_) {
-        const bool tc05 = g5_fits(M_, N_, (int)B);
-        const int64_t per = tc05 ? 512 : 256;
-        int splits = (int)((B + per - 1) / per);
-        const int cap = max_splits(M_, N_, tc05 ? SPLITS_MAX : 64);
-        splits = splits < 1 ? 1 : splits > cap ? cap : splits;
-        gemm_split(A_, lda_, 1, B_, ldb_, 0, C_, ldc_, M_, N_, (int)B, nullptr, splits, tc05 ? G5_BK : GT_K);
-    };
-    // bias gradients: column sums in two fixed-order passes (scratch: the
-    // split-K area, free between products)
-    auto colsum = [&](const float *d_, int ncol, int ld_, float *g_) {
-        int chunks = (int)((B + 127) / 128);
-        chunks = chunks > 64 ? 64 : chunks;
-        const int64_t rows_per = (B + chunks - 1) / chunks;
-        chunks = (int)((B + rows_per - 1) / rows_per);
-        colsum_part_kernel<<<dim3((unsigned)((ncol + 31) / 32), (unsigned)chunks), 256, 0, s>>>(d_, B, ncol, ld_,
-                                                                                              rows_per, part);
-        colsum_final_kernel<<<(ncol + 7) / 8, 256, 0, s>>>(part, chunks, ncol, g_);
-    };
-    // forward
-    layer1_kernel<<<ew, 256, 0, s>>>(d->x, P, z1, B);
-    silu_kernel<<<ew, 256, 0, s>>>(z1, h1, B * H);
-    gemm(h1, H, 0, P + P_W2, H, 0, z2, H, Bi, H, H, P + P_B2);
-    silu_kernel<<<ew, 256, 0, s>>>(z2, h2, B * H);
-    gemm(h2, H, 0, P + P_W3, H, 0, z3, H, Bi, H, H, P + P_B3);
-    silu_kernel<<<ew, 256, 0, s>>>(z3, h3, B * H);
-    gemm(h3, H, 0, P + P_W4, NOUT, 0, f, NOUT, Bi, NOUT, H, P + P_B4);
-    out_grad_kernel<<<148, 256, 0, s>>>(d->x, d->target, f, P, y, dd, B, d->n_fit, d->loss_part);
-    // backward
-    FFA_CHECK_CUDA(cudaMemsetAsync(G, 0, sizeof(float) * P_TOTAL, s));
-    skip_grad_kernel<<<NOUT + 16, 256, 0, s>>>(d->x, dd, B, G);
-    colsum(dd, NOUT, NOUT, G + P_BS);
-    gemm_wgrad(h3, H, dd, NOUT, G + P_W4, NOUT, H, NOUT);
-    colsum(dd, NOUT, NOUT, G + P_B4);
-    gemm(dd, NOUT, 0, P + P_W4, NOUT, 1, dh, H, Bi, H, NOUT, nullptr);
-    const float *zs[3] = {z3, z2, z1};
-    const float *hin[3] = {h2, h1, d->x};
-    const int64_t wofs[3] = {P_W3, P_W2, P_W1}, bofs[3] = {P_B3, P_B2, P_B1};
-    const int ldin[3] = {H, H, NOUT}, kin[3] = {H, H, 6};
-    for (int l = 0; l < 3; ++l) {
-        dsilu_kernel<<<ew, 256, 0, s>>>(dh, zs[l], B * H);   // dh -> dz in place
-        gemm_wgrad(hin[l], ldin[l], dh, H, G + wofs[l], H, kin[l], H);
-        colsum(dh, H, H, G + bofs[l]);
-        if (l < 2) {
-            gemm(dh, H, 0, P + wofs[l], H, 1, dz, H, Bi, H, H, nullptr);
-            float *t = dh;
-            dh = dz;
-            dz = t;
-        }
+    TrainWork w;
+    if (!train_layout(w, d->work, B)) return FFA_ERR_UNSUPPORTED;
+    AdamArgs a{d->params, d->grads, d->adam_m, d->adam_v, d->mask, d->lr, d->beta1, d->beta2, d->eps, 1.0f, 1.0f,
+               d->lr_table, d->counter, sched || d->lr > 0.0f};
+    if (!sched && a.update) {
+        a.c1 = 1.0f - powf(d->beta1, (float)d->step);
+        a.c2 = 1.0f - powf(d->beta2, (float)d->step);
     }
-    if (sched) {
-        adam_sched_kernel<<<blocks_for(P_TOTAL, 256), 256, 0, s>>>(P, G, d->adam_m, d->adam_v, P_TOTAL, d->lr_table,
-                                                                   d->counter, d->beta1, d->beta2, d->eps, d->mask);
-        counter_advance_kernel<<<1, 1, 0, s>>>(d->counter);
-    } else if (d->lr > 0.0f) {
-        const float c1 = 1.0f - powf(d->beta1, (float)d->step), c2 = 1.0f - powf(d->beta2, (float)d->step);
-        adam_kernel<<<blocks_for(P_TOTAL, 256), 256, 0, s>>>(P, G, d->adam_m, d->adam_v, P_TOTAL, d->lr, d->beta1,
-                                                             d->beta2, d->eps, c1, c2, d->mask);
-    }
+    int dev = 0, sms = 0;
+    FFA_CHECK_CUDA(cudaGetDevice(&dev));
+    FFA_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const auto tile = d->n_fit <= 4 ? train_tile_kernel<4> : train_tile_kernel<6>;
+    FFA_CHECK_CUDA(cudaFuncSetAttribute(tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT_SMEM));
+    FFA_CHECK_CUDA(cudaFuncSetAttribute(train_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TG_SMEM));
+    train_pack_kernel<<<H * H / 4 / 256, 256, 0, s>>>(d->params, w);
+    FFA_CHECK_CUDA(ffa::launch_chained(tile, (unsigned)(w.T < sms ? w.T : sms), TT_THREADS, TT_SMEM, s, d->params, d->x,
+                                       d->target, w, B, d->n_fit));
+    FFA_CHECK_CUDA(ffa::launch_chained(train_wgrad_kernel, 8 * w.S + 2 * w.SS, TG_THREADS, TG_SMEM, s, w));
+    FFA_CHECK_CUDA(ffa::launch_chained(train_update_kernel, TU_BLOCKS, 256, 0, s, w, a, d->loss_part));
     return cudaGetLastError() == cudaSuccess ? FFA_OK : FFA_ERR_CUDA;
 }
 

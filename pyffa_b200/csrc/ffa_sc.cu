@@ -47,6 +47,8 @@ namespace {
 
 namespace cg = cooperative_groups;
 using ffa::PI;
+using ffa::chain_wait;
+using ffa::launch_chained;
 
 constexpr int SC_TB = 256;
 constexpr int SC_BLOCKS = 444;             // pass1: 3 per SM on 148 SMs (one wave); fixed for determinism
@@ -68,13 +70,6 @@ struct Partial {
     double sx, sz, sx2, sz2;
     long long count;
 };
-
-// The kernels of an update follow one another by programmatic dependent launch:
-// each starts as the blocks of its predecessor exit and waits for its results
-// before it touches memory (chain_wait, no effect on an ordinary launch).
-// Letting a successor start earlier (griddepcontrol.launch_dependents) cost
-// 10-20 us of 145: its waiting blocks take the room of the running ones.
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ double py_mod(double a, double b)
 {
@@ -950,25 +945,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(solve_tb<NX>, 1)
 
 // grids the fused solve is instantiated for: square, 32 / 64 / 128
 bool fused_grid(int nx, int nz) { return nx == nz && (nx == 32 || nx == 64 || nx == 128); }
-
-// A launch that may begin while the kernel before it in the stream still runs
-// (its kernel calls chain_wait).  It hides the 1-2 us between launches: 100003
-// particles, 32 x 64 x 64 cells 52 -> 44 us.
-template <typename... P, typename... A>
-cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args)
-{
-    cudaLaunchConfig_t c = {};
-    c.gridDim = dim3(grid);
-    c.blockDim = dim3(block);
-    c.dynamicSmemBytes = smem;
-    c.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = at;
-    c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
-}
 
 template <int NX, int NZ, bool HOCK>
 cudaError_t launch_fused_t(const unsigned long long *acc, const SCState *st, int ns, const float *gk, float *rho,
