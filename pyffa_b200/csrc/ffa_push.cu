@@ -419,9 +419,8 @@ __device__ __forceinline__ double3 rf_spiral64(const RFK &rf, double acc, double
     return make_double3((acc * er) * s, ((acc * ez) * z) * s, (acc * ef) * s);   // Er, Ez, Efi
 }
 
-// Er, Efi of fixed gap g at a particle inside its angular window (out of
-// line: a few steps of a turn come here)
-__device__ __noinline__ double2 gap_field64(const RFK &rf, int g, double acc, double r, double fi, double rfph)
+// Er, Efi of fixed gap g at a particle inside its angular window
+__device__ __forceinline__ double2 gap_field(const RFK &rf, int g, double acc, double r, double fi, double rfph)
 {
     double sf, cf;
     sincos(fi, &sf, &cf);
@@ -430,6 +429,17 @@ __device__ __noinline__ double2 gap_field64(const RFK &rf, int g, double acc, do
     sincos(rf.theta_n[g] - fi, &sd, &cd);
     const double s = sin(rfph + rf.rf_shift[g]);
     return make_double2((acc * cd) * s, (acc * sd) * s);
+}
+
+// The FP64 kernels call their rare branches out of line (a few steps of a turn
+// come there), which keeps the usual step short.  The FP32C kernels, at 80
+// registers with spills, have no registers to spare around a call and keep
+// them inline: with the calls FP32C RK4 took 7 % and FP32C Boris with space
+// charge 14 % longer (5.48 against 5.11 ms per 360 steps of 1e5 particles,
+// 1.94 against 1.71 ms per 60 steps of 1e6).
+__device__ __noinline__ double2 gap_field64(const RFK &rf, int g, double acc, double r, double fi, double rfph)
+{
+    return gap_field(rf, g, acc, r, fi, rfph);
 }
 
 // RF field (cylindrical r, z, fi components) times sin(RF phase +
@@ -453,7 +463,7 @@ __device__ __forceinline__ void rf_field64(const RFK &rf, double acc, double r, 
     const int g0 = rf.physical_sum ? 0 : rf.ngaps - 1;
     for (int g = g0; g < rf.ngaps; ++g) {
         if (!in_window(rf, g, fi)) continue;
-        const double2 e = gap_field64(rf, g, acc, r, fi, rfph);
+        const double2 e = gap_field(rf, g, acc, r, fi, rfph);
         Er += e.x;
         Efi += e.y;
     }
@@ -484,7 +494,7 @@ __device__ __forceinline__ bool rf_hit64(const RFK &rf, const double *acc, doubl
     return e.x != 0.0 || e.y != 0.0 || e.z != 0.0;
 }
 
-__device__ __noinline__ double3 wide_rotation(double y, double x)
+__device__ __forceinline__ double3 atan_rotation(double y, double x)
 {
     const double a = atan2(y, x);
     double s, c;
@@ -492,12 +502,15 @@ __device__ __noinline__ double3 wide_rotation(double y, double x)
     return make_double3(a, s, c);
 }
 
+__device__ __noinline__ double3 wide_rotation(double y, double x) { return atan_rotation(y, x); }
+
 // Azimuth change of one step and its sine / cosine, from the new position's
 // unit vector in the local frame: sin and cos of the step angle are y / r and
 // x / r (r^-1 is at hand from the drift); a step turns the particle by about
 // 2 pi / (steps per turn), and for |sin| < 0.02 the angle is the arcsine series
 //   asin(s) = s (1 + s^2/6 + 3 s^4/40 + 5 s^6/112 + 35 s^8/1152)
 // (truncation < 3e-19 relative): no division and no sin/cos series.
+template <bool INLINE = false>
 __device__ __forceinline__ void step_rotation(double y, double x, double ir, double &a, double &s, double &c)
 {
     const double s0 = y * ir;
@@ -507,7 +520,7 @@ __device__ __forceinline__ void step_rotation(double y, double x, double ir, dou
         s = s0;
         c = x * ir;
     } else {
-        const double3 w = wide_rotation(y, x);
+        const double3 w = INLINE ? atan_rotation(y, x) : wide_rotation(y, x);
         a = w.x;
         s = w.y;
         c = w.z;
@@ -675,8 +688,15 @@ struct SCExtrap {
     // ph: the step's position gs mod sc_step in its interval (0 in the first)
     __device__ void apply(int ph, double inv_sc, double &esr, double &esz, double &esf) const
     {
-        if (!pre) return;
-        const double sf = (double)ph * inv_sc;
+        if (pre) blend((double)ph * inv_sc, esr, esz, esf);
+    }
+    // FP32C: the fraction formed anew from the step number
+    __device__ void apply(const PushK &p, int64_t gs, double &esr, double &esz, double &esf) const
+    {
+        if (pre) blend(gs >= p.sc_step ? (double)(gs % p.sc_step) / (double)p.sc_step : 0.0, esr, esz, esf);
+    }
+    __device__ void blend(double sf, double &esr, double &esz, double &esf) const
+    {
         if (pp) {
             esr = epr + sf * (epr - eqr);
             esz = epz + sf * (epz - eqz);
@@ -1010,7 +1030,7 @@ __global__ void __maxnreg__(NREG) boris_f32c_kernel(const __grid_constant__ Push
     for (int s = 0; s < p.nsteps; ++s) {
         const int64_t gs = p.step0 + s;
         if (injs == gs) { inj = 1; surv = 1; }
-        if (SC) ex.apply(sc_phase(p, gs), p.inv_sc, esr, esz, esf);
+        if (SC) ex.apply(p, gs, esr, esz, esf);
         const double drf = __ldg(p.drf + gs);
         double pre[7];
         const int surv0 = surv;
@@ -1070,7 +1090,7 @@ __global__ void __maxnreg__(NREG) boris_f32c_kernel(const __grid_constant__ Push
             const double irn = rsqrt(rr2);
             const double rn = rr2 * irn;
             double dfi, sn, cn;
-            step_rotation(yn, xn, irn, dfi, sn, cn);
+            step_rotation<true>(yn, xn, irn, dfi, sn, cn);
             fi = fi + dfi;
             rdot = vxn * cn + vyn * sn;
             const double vfi = -vxn * sn + vyn * cn;
@@ -1507,7 +1527,7 @@ __global__ void __maxnreg__(80) rk4_f32c_kernel(const __grid_constant__ PushK p)
     for (int s = 0; s < p.nsteps; ++s) {
         const int64_t gs = p.step0 + s;
         if (injs == gs) { inj = 1; surv = 1; }
-        if (SC) ex.apply(sc_phase(p, gs), p.inv_sc, esr, esz, esf);
+        if (SC) ex.apply(p, gs, esr, esz, esf);
         const double *rate = p.drf + 4 * gs;
         const double *acc = p.acc + 4 * gs;
         const double k1rf = h * __ldg(rate + 0), k2rf = h * __ldg(rate + 1);
