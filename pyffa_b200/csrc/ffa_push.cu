@@ -840,8 +840,8 @@ __device__ __forceinline__ void field_mixed(const FieldK &f, double r, double ir
 // Large bunches are bound by the L1 data pipe (z_taylor64), small ones by one
 // step's chain: the node loads from L2 (about 300 cycles) and some 110
 // dependent FP64 operations of 8 cycles.  720 steps, with the tables of field64
-// and the planes of z_taylor64: 1e5 particles, order 2, RF 2.47 -> 1.54 ms; 1e4
-// particles, order 4, 1.88 -> 0.79 ms; 1e6 particles, 60 steps with space
+// and the planes of z_taylor64: 1e5 particles, order 2, RF 2.47 -> 1.42 ms; 1e4
+// particles, order 4, 1.88 -> 0.77 ms; 1e6 particles, 60 steps with space
 // charge 2.05 -> 1.69 ms.
 template <int MAXO, bool SC, bool XING, int NREG, bool HARM = false>
 __global__ void __maxnreg__(NREG) boris_f64_kernel(const __grid_constant__ PushK p)
@@ -1745,12 +1745,15 @@ cudaError_t launch_pack_nodes(const ffa_field_desc &d, int npad, double *n64, fl
 // keep more of a step's loads and chains in flight per warp, fewer hold more
 // warps; 80, 128 and 255 leave 24, 16 and 8 warps per SM.  What decides is how
 // many waves the warps make (us per 180 steps, z-Taylor order 2, RF, 148 SMs):
-//   particles     10000  56800  75000  100000  113600  150000  300000  1000000
-//   80 registers    252    276    303     375     376     610     980     2971
-//   128 registers   199    221    254     418     431     480     929     2996
-//   255 registers   198    219    405     417     425     605    1162     3608
-// so 128 up to 16 warps per SM, 80 while that is one wave, and 128 again
-// beyond.  From order 3 a step's node loads alone need more than 128 (order 4,
+//   particles     10000  56800  75000  100000  113600  150000  200000  300000  1000000
+//   80 registers    246    268    281     357     355     570     623     908     2739
+//   128 registers   197    218    252     421     434     480     657     929     3001
+//   255 registers   198    219    405     417     425     605       -    1162     3608
+// so 128 up to 16 warps per SM, 80 while that is one wave, 128 again while that
+// is two, and 80 beyond (order 0, 120 steps, 1e6 particles: 1338 us with 128,
+// 1113 with 80; order 1 1754 and 1486).  Orders 3 and 4 stay at 128 there (order
+// 4, 300000 particles: 830 us, with 80 901; 1e6: 2745 and 2700), and so do the
+// launches that look for crossings, which hold more values over a step.  From order 3 a step's node loads alone need more than 128 (order 4,
 // 10000 particles, 720 steps: 935 us with 128, 791 us with 255).  With space
 // charge the endpoints' registers make 80 spill (60 steps, 1e6 particles: 1898
 // us, 1627 us with 128; 100000: 227 and 224).
@@ -1762,7 +1765,8 @@ static int boris_cap(const PushK &p, bool sc, int max_order)
     const int64_t warps = (p.n + 31) / 32;
     if (max_order >= 3 && warps <= (int64_t)8 * sms) return 255;
     if (warps <= (int64_t)16 * sms) return 128;
-    return warps <= (int64_t)24 * sms ? 80 : 128;
+    if (warps <= (int64_t)24 * sms) return 80;
+    return max_order >= 3 || xing_on(p) || warps <= (int64_t)32 * sms ? 128 : 80;
 }
 
 template <int MAXO, bool SC, int NREG, bool HARM>
