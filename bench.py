@@ -39,7 +39,7 @@ MAX_ORDER = 2
 FP64_FLOP_PER_PARTICLE_STEP = 300.0
 # the kernel's executed float64 operations per particle-step (2 per DFMA, 1
 # per DADD / DMUL), counted by ncu on this workload: reported beside it
-FP64_EXEC_FLOP_PER_PARTICLE_STEP = 419.4
+FP64_EXEC_FLOP_PER_PARTICLE_STEP = 213.7
 # algorithmic float64 operations per particle-step of one RK4 step: four
 # right-hand sides (azimuth mod sector 3, analytic field 93, z-Taylor sum 77,
 # RF window test 4, equations of motion 40) and the stage arithmetic (k = h d,
@@ -48,7 +48,7 @@ FP64_EXEC_FLOP_PER_PARTICLE_STEP = 419.4
 RK4_FLOP_PER_PARTICLE_STEP = 980.0
 # DRAM bytes (read + write) of one launch (one turn, 1e5 particles) from an
 # ncu capture of the same launch, L2 flushed before it
-BORIS_TRAFFIC_PER_LAUNCH = 19.571e6
+BORIS_TRAFFIC_PER_LAUNCH = 17.443e6
 # algorithmic HBM bytes per particle per launch: SoA state read
 # (10 float64 + 2 flag bytes + int32 injection step) and written (10 float64 + 2 bytes)
 STATE_BYTES_PER_PARTICLE = (10 * 8 + 2 + 4) + (10 * 8 + 2)

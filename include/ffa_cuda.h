@@ -534,8 +534,8 @@ int ffa_mlp_train_step(const ffa_mlp_train_desc *desc, void *stream);
 int ffa_mlp_gemm(const float *A, int lda, int transA, const float *B, int ldb, int transB, float *C, int ldc,
                  int M, int N, int K, const float *bias, void *stream);
 
-/* Tensor-core GEMM tiles (ffa_mlp_gemm, ffa_mlp_train_step) whose bounded
- * pipeline waits ran out since the last call (their output tiles hold NaN);
+/* Tiles of ffa_mlp_gemm and ffa_mlp_train_step whose bounded pipeline waits
+ * ran out since the last call (their outputs, loss or gradients hold NaN);
  * reads and clears the device counter, synchronising the device.  No
  * counterpart in the reference (its training path does not exist; the
  * learned map is new). */

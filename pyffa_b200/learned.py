@@ -461,7 +461,7 @@ class Trainer:
     lr_table (device float32, one learning rate per step) switches to the
     device schedule: step k takes lr_table[k] and Adam's bias corrections of
     step k + 1 from a device counter, so that graph_step can replay one
-    captured CUDA graph of the whole step (about 30 launches) with nothing
+    captured CUDA graph of the whole step (four kernels) with nothing
     read from the host; step() then ignores its lr argument."""
 
     def __init__(self, params, batch=8192, n_fit=4, freeze_skip=True, beta1=0.9, beta2=0.999, eps=1e-8,

@@ -143,8 +143,8 @@ class Pusher:
     particle range pushed and recomputed every `order_every` launches of
     that range (0: never), so that a warp's z-Taylor node loads share cache
     lines; None -- thread t advances particle t; "auto" (default) -- morton
-    for the float64 pushers, whose time goes to those loads (c1 Boris: 2.64
-    -> 2.47 ms per 1e5-particle turn; 1e6 particles: 23.9 -> 18.7 ms), None
+    for the float64 pushers, whose time goes to those loads (c1 Boris: 2.17
+    -> 1.37 ms per 1e5-particle turn; 1e6 particles: 20.9 -> 10.9 ms), None
     for the float32-field ones (no gain measured).  The results are the same
     either way.  Ranges under `order_min` particles keep the identity."""
 
