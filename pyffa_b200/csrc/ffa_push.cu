@@ -1380,7 +1380,7 @@ __global__ void __maxnreg__(NREG) rk4_f64_kernel(const __grid_constant__ PushK p
     SCExtrap ex;
     if (SC) ex.load(S, i);
     const double h = p.dt, h6 = p.dt * (1.0 / 6.0), c2 = p.cs.c * p.cs.c, q = p.cs.q;
-    double Ev = 0.0, v2 = 0.0, qc2E = 0.0;       // the energy these two belong to
+    double Ev = __longlong_as_double(0x7FF8000000000000ll), v2 = 0.0, qc2E = 0.0;   // the energy these two belong to (none yet)
     int oob = 0;
     for (int s = 0; s < p.nsteps; ++s) {
         const int64_t gs = p.step0 + s;
@@ -1409,7 +1409,9 @@ __global__ void __maxnreg__(NREG) rk4_f64_kernel(const __grid_constant__ PushK p
                     qc2E = q * c2 * iE;
                 }
                 const double vp2 = v2 - yvr * yvr - yvz * yvz;
-                const double vp = vp2 * rsqrt64(vp2);
+                // rsqrt64 wants a normal argument: a particle at rest, or moving
+                // in r and z alone, has vp2 == 0 and vp = 0 (negative: NaN)
+                const double vp = vp2 == 0.0 ? 0.0 : vp2 * rsqrt64(vp2);
                 const double w = vp * ir;                        // d(fi)/dt
                 double dvr = vp * w + qc2E * (yvz * Bfi - vp * Bz);
                 double dvz = qc2E * (vp * Br - yvr * Bfi);

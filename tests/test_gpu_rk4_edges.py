@@ -1,0 +1,66 @@
+"""FP64 RK4 at the ends of its arithmetic, against the oracle: a live particle
+at rest (E equal to E0, no velocity: the azimuthal velocity is the root of an
+exact 0) and one without any energy, which the equations of motion make NaN."""
+import os
+import tempfile
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("CUDA device required")
+
+
+def machine(k=7.6, B0=None, order=0):
+    from pyffa_b200 import synthetic
+    from pyffa_b200.constants import FFAG_GlobalParameters
+    from pyffa_b200.fields import FFAG_Bfield_analytical, FFAG_EField_new
+    cfg = synthetic.lattice_bmap(r_range=(8.0, 9.3, 0.01), theta_step_deg=0.05)
+    cfg["Bmap"]["coefficients_tupel"] = [1.6 / 8.6 ** k if B0 is None else B0, k]
+    bm = FFAG_Bfield_analytical(config=cfg, max_order=order, AddNumricalMap=False)
+    em = FFAG_EField_new(synthetic.emap_file(os.path.join(tempfile.mkdtemp(), "emap.txt")), EnableFlag=False)
+    gp = FFAG_GlobalParameters()
+    gp.AddBMap(bm)
+    gp.AddEMap(em)
+    return bm, em, gp
+
+
+def rows(n):
+    from pyffa_b200 import synthetic
+    from pyffa_b200.constants import FFAG_ConversionTools
+    v = FFAG_ConversionTools().ConvertPrzek2Vrzek(synthetic.gaussian_bunch(n, seed=4))
+    v[:, 7] = v[:, 8] = 1.0
+    return v
+
+
+def step(gp, v, dt):
+    from pyffa_b200.track import FFAG_RungeKutta
+    return v + FFAG_RungeKutta().rk4_step_malloc(None, 0.0, v, dt, gp)[0]
+
+
+def test_particles_at_rest_and_without_energy():
+    from oracle import oracle as O
+    from pyffa_b200 import synthetic
+    from pyffa_b200.constants import E0_J
+    bm, em, gp = machine()
+    v = rows(40)
+    v[3, 1] = v[3, 3] = 0.0
+    v[3, 5] = E0_J
+    v[17, 1] = v[17, 3] = 0.0
+    v[17, 5] = 0.0
+    dt = synthetic.steps_per_turn_dt(steps_per_turn=720)
+    ref = v.copy()
+    O.track(O.Setup(bm, em, gp), "RK4", ref, 0.0, dt, 1)
+    got = step(gp, v, dt)
+    assert np.array_equal(ref[3, :6], v[3, :6]) and np.array_equal(got[3, :6], v[3, :6])   # it stays where it is
+    assert np.isnan(ref[17, :5]).all() and np.isnan(got[17, :5]).all()
+    rest = np.delete(np.arange(40), [3, 17])
+    # one step of ~100 operations: see the one-step bound of the field-table test
+    for c in range(6):
+        assert np.max(np.abs(got[rest, c] - ref[rest, c])) <= 1e-14 * np.abs(ref[rest, c]).max(), c
