@@ -220,6 +220,10 @@ void field_tables(FieldK &k, std::vector<double> &tab)
         }
     }
     if (k.pw_n == 0) tab.insert(tab.end(), 2, 0.0);
+    if (k.k == 0.0) {                                // no power: every r is inside a one-entry table of zeros
+        k.pw_n = 1;
+        k.pw_scale = 0.0;
+    }
 }
 
 }  // namespace

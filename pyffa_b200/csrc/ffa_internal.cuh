@@ -89,6 +89,7 @@ struct FieldK {
     // Power table: (B0 r_j^(k-1), 1 / r_j) at r_j = (pw_j0 + j) pw_h,
     // pw_h = 1 / pw_scale = 2^-p m, and the binomial coefficients 1 .. 4 of
     // the exponent k - 1; without a table one dummy entry that no r reaches
+    // (k = 0: that every r reaches, pw_scale = 0)
     int32_t pw_j0, pw_n;
     double pw_scale, pw_h;
     const double2 *pw_tab;

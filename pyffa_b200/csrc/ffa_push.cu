@@ -211,12 +211,13 @@ __device__ __forceinline__ Tables tables_fetch(const FieldK &f, double ri, doubl
     return t;
 }
 
-// F, F', B0 r^(k-1) and its k-fold from the entries of a point
+// F, F', B0 r^k and k B0 r^(k-1) from the entries of a point
 __device__ __forceinline__ void tables_eval(const FieldK &f, const Tables &t, double ri, double &F, double &Fp,
-                                            double &G, double &kG)
+                                            double &B0r, double &kG)
 {
     flutter_eval(f, t.fl, F, Fp);
-    G = power_eval(f, t.pw, ri);
+    const double G = power_eval(f, t.pw, ri);
+    B0r = G * ri;
     kG = f.k * G;
     if (f.unusual) {                     // no flutter table, or a field index of 0
         if (f.fl_direct) {
@@ -224,7 +225,10 @@ __device__ __forceinline__ void tables_eval(const FieldK &f, const Tables &t, do
             F = v.x;
             Fp = v.y;
         }
-        if (f.k == 0.0) G = f.B0 / ri;
+        if (f.k == 0.0) {                // B0 at every radius, also at r <= 0
+            B0r = f.B0;
+            kG = 0.0;
+        }
     }
 }
 
@@ -327,9 +331,9 @@ __device__ __forceinline__ void field64(const FieldK &f, double r, double ir, do
     if constexpr (MAXO >= 1) cell = map_cell(f, r, fim, clamped);
     const Tables t = tables_fetch(f, r, fim);
     if constexpr (MAXO >= 1) z_taylor64<MAXO>(f, cell, z, hz, hf, hr);
-    double F, Fp, G, kG;
-    tables_eval(f, t, r, F, Fp, G, kG);
-    const double B0r = G * r, B0Fp = B0r * Fp;
+    double F, Fp, B0r, kG;
+    tables_eval(f, t, r, F, Fp, B0r, kG);
+    const double B0Fp = B0r * Fp;
     Bz = fma(B0r, F, hz);
     Bfi = fma(B0Fp, ir, hf) * z;
     Br = (fma(kG, F, hr) - B0Fp * t.spiral_p) * z;
@@ -1603,16 +1607,16 @@ __device__ __forceinline__ double sector_azimuth(const FieldK &f, double t)
 }
 
 // d/dtheta of (r, pr, z, pz) at fixed momentum P (FunctionForSEO,
-// src/FFAG_track.py:1698-1740), qP = q / P, from the flutter F, F', G = B0
-// r^(k-1) and kG = k G.  The field enters only times r, which cancels the 1 / r
-// of Bfi.
-__device__ __forceinline__ void seo_rhs(const double x[4], double qP, double F, double Fp, double G, double kG,
+// src/FFAG_track.py:1698-1740), qP = q / P, from the flutter F, F', B0r = B0
+// r^k and kG = k B0 r^(k-1).  The field enters only times r, which cancels the
+// 1 / r of Bfi.
+__device__ __forceinline__ void seo_rhs(const double x[4], double qP, double F, double Fp, double B0r, double kG,
                                         double spiral_p, double d[4])
 {
     const double r = x[0], pr = x[1], z = x[2], pz = x[3];
     const double pf2 = 1.0 - pr * pr - pz * pz, ipf = rsqrt64(pf2);
-    const double Gr = G * r, rBz = Gr * r * F, rBfi = Gr * Fp * z;
-    const double rBr = r * fma(kG, F, -Gr * Fp * spiral_p) * z;
+    const double rBz = B0r * r * F, rBfi = B0r * Fp * z;
+    const double rBr = r * fma(kG, F, -B0r * Fp * spiral_p) * z;
     const double ur = pr * ipf, uz = pz * ipf;
     d[0] = r * ur;
     d[1] = fma(pf2, ipf, qP * (uz * rBfi - rBz));
@@ -1676,12 +1680,12 @@ __global__ void __launch_bounds__(32) theta_track_kernel(const __grid_constant__
         auto rhs = [&](double ts, const double *y, double F, double Fp, double *k) {
             if constexpr (PLAIN) {
                 const double G = power_eval(f, power_fetch(f, y[0]), y[0]);
-                seo_rhs(y, qP, F, Fp, G, f.k * G, 0.0, k);
+                seo_rhs(y, qP, F, Fp, G * y[0], f.k * G, 0.0, k);
             } else {
                 const Tables tab = tables_fetch(f, y[0], sector_azimuth(f, ts));
-                double G, kG;
-                tables_eval(f, tab, y[0], F, Fp, G, kG);
-                seo_rhs(y, qP, F, Fp, G, kG, tab.spiral_p, k);
+                double B0r, kG;
+                tables_eval(f, tab, y[0], F, Fp, B0r, kG);
+                seo_rhs(y, qP, F, Fp, B0r, kG, tab.spiral_p, k);
             }
         };
         double y[4], k[4], S[4];

@@ -1,6 +1,7 @@
 """FP64 RK4 at the ends of its arithmetic, against the oracle: a live particle
 at rest (E equal to E0, no velocity: the azimuthal velocity is the root of an
-exact 0) and one without any energy, which the equations of motion make NaN."""
+exact 0), one without any energy, which the equations of motion make NaN, and
+the field of index 0, which is B0 at every radius, at radii of either sign."""
 import os
 import tempfile
 
@@ -64,3 +65,21 @@ def test_particles_at_rest_and_without_energy():
     # one step of ~100 operations: see the one-step bound of the field-table test
     for c in range(6):
         assert np.max(np.abs(got[rest, c] - ref[rest, c])) <= 1e-14 * np.abs(ref[rest, c]).max(), c
+
+
+def test_field_index_zero_at_any_radius():
+    """The equations of motion are defined at r < 0 (fi' = v / r), and a field
+    of index 0 does not depend on r."""
+    from oracle import oracle as O
+    from pyffa_b200 import synthetic
+    bm, em, gp = machine(k=0.0, B0=1.6)
+    v = rows(64)
+    v[:, 0] = np.r_[-np.geomspace(1e-3, 9.0, 32), np.geomspace(1e-3, 9.0, 32)]
+    v[:, 4] = np.random.default_rng(2).uniform(0, 2 * np.pi / 12, 64)
+    dt = 1e-15                        # 0.3 um: the azimuth turns by at most 3e-4 rad at 1 mm
+    ref = v.copy()
+    O.track(O.Setup(bm, em, gp), "RK4", ref, 0.0, dt, 1)
+    got = step(gp, v, dt)
+    assert np.isfinite(ref[:, :6]).all() and np.isfinite(got[:, :6]).all()
+    for c in range(6):
+        assert np.max(np.abs(got[:, c] - ref[:, c])) <= 1e-14 * np.abs(ref[:, c]).max(), c
