@@ -1409,7 +1409,9 @@ __global__ void __maxnreg__(NREG) rk4_f64_kernel(const __grid_constant__ PushK p
                 field64<MAXO>(f, yr, ir, fim, yz, Bz, Br, Bfi, oob);
                 if constexpr (HARM) Bz += harmonics_bz(f.harm, f.n_harm, yr, yfi);
                 if (yE != Ev) {
-                    const double iE = 1.0 / yE, ig = p.cs.E0 * iE;
+                    // ig = E0 / E, the product corrected by its residual: at low
+                    // energies its rounding is divided by beta^2 in v2
+                    const double iE = 1.0 / yE, ig0 = p.cs.E0 * iE, ig = fma(fma(-ig0, yE, p.cs.E0), iE, ig0);
                     Ev = yE;
                     v2 = (1.0 - ig * ig) * c2;
                     qc2E = q * c2 * iE;

@@ -1,7 +1,8 @@
 """FP64 RK4 at the ends of its arithmetic, against the oracle: a live particle
 at rest (E equal to E0, no velocity: the azimuthal velocity is the root of an
 exact 0), one without any energy, which the equations of motion make NaN, and
-the field of index 0, which is B0 at every radius, at radii of either sign."""
+the field of index 0, which is B0 at every radius, at radii of either sign; and
+the speed at low energies, where E0 / E is close to 1."""
 import os
 import tempfile
 
@@ -83,3 +84,26 @@ def test_field_index_zero_at_any_radius():
     assert np.isfinite(ref[:, :6]).all() and np.isfinite(got[:, :6]).all()
     for c in range(6):
         assert np.max(np.abs(got[:, c] - ref[:, c])) <= 1e-14 * np.abs(ref[:, c]).max(), c
+
+
+def test_speed_at_low_energies():
+    """A straight line from its perigee: the azimuth advances by atan(v h / r).
+    v^2 = c^2 (1 - (E0 / E)^2) divides the rounding of E0 / E, half an ulp of a
+    number below 1 (2^-54), by beta^2: 2^-54 / beta^2 of v, half as much again
+    for a square that is not fused, and ~16 ulp for the rest of the step (its
+    truncation at 1e-4 rad is below 1e-16)."""
+    from pyffa_b200.constants import C_LIGHT, E0_J, E0_MEV
+    _, _, gp = machine(k=7.6, B0=0.0)
+    n = 20_000
+    v = rows(n)
+    v[:, 0] = 8.5
+    v[:, 1:5] = 0.0
+    v[:, 5] = E0_J * (1 + np.random.default_rng(7).uniform(0.5, 10.0, n) / E0_MEV)
+    ig = np.longdouble(E0_J) / v[:, 5].astype(np.longdouble)
+    beta2 = 1 - ig * ig
+    speed = np.longdouble(C_LIGHT) * np.sqrt(beta2)
+    h = 1e-4 * 8.5 / float(speed.max())
+    got = step(gp, v, h)[:, 4]
+    ref = np.arctan(speed * np.longdouble(h) / np.longdouble(8.5))
+    err = np.abs(got / ref - 1).astype(np.float64)
+    assert (err <= 1.5 * 2.0 ** -54 / beta2.astype(np.float64) + 16 * 2.0 ** -53).all(), (err * beta2 * 2.0 ** 54).max()
