@@ -3,6 +3,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <new>
 #include <vector>
 
 #include "ffa_internal.cuh"
@@ -302,7 +303,12 @@ int ffa_fieldmap_create(const ffa_field_desc *d, void *stream, ffa_fieldmap **ou
     for (int j = 0; j < d->n_convex; ++j) k.seg_yk[j] = k.seg_y[j] * k.seg_k[j];
     {
         std::vector<double> tab;
-        field_tables(k, tab);
+        try {
+            field_tables(k, tab);
+        } catch (const std::bad_alloc &) {          // nothing is thrown through the C entry
+            free(fm);
+            return FFA_ERR_NOMEM;
+        }
         k.unusual = k.fl_direct || k.k == 0.0;
         if (cudaMalloc(&fm->tables, sizeof(double) * tab.size()) != cudaSuccess) {
             free(fm);
