@@ -227,6 +227,24 @@ void field_tables(FieldK &k, std::vector<double> &tab)
     }
 }
 
+// The tables' device copy, made outside the caller's streams: a mid-plane map
+// asks nothing of them, so it can be made while one is captured (allocations are
+// then refused unless the thread's capture mode is relaxed) and waits for none.
+cudaError_t upload_tables(const double *tab, size_t bytes, double **out)
+{
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return e;
+    cudaStream_t s = nullptr;
+    e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMalloc(out, bytes);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(*out, tab, bytes, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (s) cudaStreamDestroy(s);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return e;
+}
+
 }  // namespace
 
 extern "C" {
@@ -310,16 +328,16 @@ int ffa_fieldmap_create(const ffa_field_desc *d, void *stream, ffa_fieldmap **ou
             return FFA_ERR_NOMEM;
         }
         k.unusual = k.fl_direct || k.k == 0.0;
-        if (cudaMalloc(&fm->tables, sizeof(double) * tab.size()) != cudaSuccess) {
-            free(fm);
-            return FFA_ERR_NOMEM;
-        }
-        if (cudaMemcpy(fm->tables, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        const cudaError_t e = upload_tables(tab.data(), sizeof(double) * tab.size(), &fm->tables);
+        // a mid-plane map can be described where there is no device to push on
+        // (FFA_ERR_CUDA from the calls that would read its tables)
+        const bool absent = e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver;
+        if (e != cudaSuccess && !(absent && d->max_order == 0)) {
             ffa_fieldmap_destroy(fm);
-            return FFA_ERR_CUDA;
+            return e == cudaErrorMemoryAllocation || absent ? FFA_ERR_NOMEM : FFA_ERR_CUDA;
         }
         k.fl_tab = fm->tables;
-        k.pw_tab = reinterpret_cast<const double2 *>(fm->tables + 8 * (size_t)k.fl_n);
+        k.pw_tab = fm->tables ? reinterpret_cast<const double2 *>(fm->tables + 8 * (size_t)k.fl_n) : nullptr;
     }
     if (d->max_order > 0) {
         const int64_t plane = d->r_size * d->fi_size;
@@ -412,6 +430,7 @@ static int push_impl(const ffa_fieldmap *fm, const ffa_rf_desc *rf, const ffa_ap
     if (nreg_sel && (!(flags & FFA_FP32C) || (sc_step > 0 && st->sc_pre) || fm->k.n_harm > 0))
         return FFA_ERR_UNSUPPORTED;
     if (n == 0 || nsteps == 0) return FFA_OK;
+    if (!fm->tables) return FFA_ERR_CUDA;            // made without a device
 
     PushK p;
     memset(&p, 0, sizeof(p));
@@ -527,6 +546,7 @@ int ffa_theta_track(const ffa_fieldmap *fm, const ffa_theta_track_desc *d, void 
     if (d->time_mode != 0 && d->time_mode != 1) return FFA_ERR_INVALID;
     if (d->traj && d->traj_cols != 2 && d->traj_cols != 7) return FFA_ERR_INVALID;
     if (d->m == 0) return FFA_OK;
+    if (!fm->tables) return FFA_ERR_CUDA;            // made without a device
     return launch_theta_track(fm->k, *d, as_stream(stream)) == cudaSuccess ? FFA_OK : FFA_ERR_CUDA;
 }
 

@@ -1,6 +1,9 @@
-"""ffa_fieldmap_create on the host: its errors come back as codes."""
+"""ffa_fieldmap_create on the host: its errors come back as codes, and a
+mid-plane map (no node tables) can be made without a device."""
 import subprocess
 import sys
+
+import pytest
 
 from pyffa_b200 import build
 
@@ -32,3 +35,11 @@ def create(fringe, room=0):
 def test_no_room_for_the_tables_is_an_error_code():
     # a sharp fringe's flutter table takes 4.4 MB; the process has 2 MB left
     assert create(0.0035, 2 << 20) == (3, 0)          # FFA_ERR_NOMEM
+
+
+def test_mid_plane_map_without_a_device():
+    torch = pytest.importorskip("torch")
+    if torch.cuda.is_available():
+        pytest.skip("there is a device")
+    assert create(0.19) == (0, 1)
+    assert create(0.0035) == (0, 1)
