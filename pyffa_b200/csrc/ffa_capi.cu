@@ -114,18 +114,76 @@ unsigned blocks_for(int64_t n, int tb) { return (unsigned)((n + tb - 1) / tb); }
 
 // ------------------------------------------- one-dimensional field tables
 //
-// Taylor coefficients 0 .. N-1 of the logistic sigma(u0 + s x) in x, by the
-// recurrence of sigma' = sigma (1 - sigma):
+// Taylor coefficients of the logistic sigma(u0 + s x) in x, by the recurrence of
+// sigma' = sigma (1 - sigma):
 //   (n + 1) c_(n+1) = s (c_n - sum_i c_i c_(n-i)).
+// Orders 0 to 2 in long double; from order 3, where a cell's terms (|s| <= 0.04,
+// |x| <= 1/2) are below 2e-7 of F, double rounds by less than 1e-22.
 constexpr int FL_SERIES = 12;
 
-void logistic_series(long double u0, long double s, long double c[FL_SERIES])
+struct Series {
+    long double l[3];
+    double c[FL_SERIES];
+    bool flat;                          // orders above 0 vanish
+};
+
+void logistic_series(long double c0, long double s, Series &t)
 {
-    c[0] = 1.0L / (1.0L + expl(-u0));
-    for (int n = 0; n + 1 < FL_SERIES; ++n) {
+    t.l[0] = c0 < 1e-280L ? 0.0L : c0;  // (the tail's end, clear of denormal numbers)
+    t.flat = t.l[0] == 0.0L || t.l[0] == 1.0L;
+    if (t.flat) return;
+    t.l[1] = s * (c0 - c0 * c0);
+    t.l[2] = s * (t.l[1] - 2.0L * c0 * t.l[1]) / 2.0L;
+    for (int n = 0; n < 3; ++n) t.c[n] = (double)t.l[n];
+    if (c0 < 0x1p-70L) {                // the exponential tail: the products are lost beside c_n
+        for (int n = 2; n + 1 < FL_SERIES; ++n) t.c[n + 1] = (double)s * t.c[n] * (1.0 / (n + 1));
+        return;
+    }
+    const double d = (double)(1.0L - 2.0L * c0), sd = (double)s;
+    for (int n = 2; n + 1 < FL_SERIES; ++n) {
+        double q = 0.0;                 // the pairs i, n - i twice, the latest last
+        for (int i = (n - 1) / 2; i >= 1; --i) q += t.c[i] * t.c[n - i];
+        q = d * t.c[n] - 2.0 * q;
+        if (n % 2 == 0) q -= t.c[n / 2] * t.c[n / 2];
+        t.c[n + 1] = sd * q * (1.0 / (n + 1));
+    }
+}
+
+// One edge of a magnet, cell by cell: sigma of u = u0 + j s.  exp(-u) is carried
+// from cell to cell and formed anew every 16th (16 roundings of 2^-64).
+struct Edge {
+    long double u0, s, step, e;
+    Edge(long double u0_, long double s_) : u0(u0_), s(s_), step(expl(-s_)), e(0.0L) {}
+    void at(int j, Series &t)
+    {
+        e = j & 15 ? e * step : expl(-(u0 + (long double)j * s));
+        logistic_series(1.0L / (1.0L + e), s, t);
+    }
+};
+
+// Adds y a b to the orders l (0 to 2) and c (3 on)
+void add_product(double y, const Series &a, const Series &b, long double l[3], double c[FL_SERIES])
+{
+    if (a.flat && b.flat) {
+        l[0] += (long double)y * (a.l[0] * b.l[0]);
+        return;
+    }
+    if (a.flat || b.flat) {             // by exactly 0 or 1
+        const Series &f = a.flat ? a : b, &v = a.flat ? b : a;
+        if (f.l[0] == 0.0L) return;
+        for (int n = 0; n < 3; ++n) l[n] += (long double)y * v.l[n];
+        for (int n = 3; n < FL_SERIES; ++n) c[n] += y * v.c[n];
+        return;
+    }
+    for (int n = 0; n < 3; ++n) {
         long double q = 0.0L;
-        for (int i = 0; i <= n; ++i) q += c[i] * c[n - i];
-        c[n + 1] = s * (c[n] - q) / (long double)(n + 1);
+        for (int i = 0; i <= n; ++i) q += a.l[i] * b.l[n - i];
+        l[n] += (long double)y * q;
+    }
+    for (int n = 3; n < FL_SERIES; ++n) {
+        double q = 0.0;
+        for (int i = 0; i <= n; ++i) q += a.c[i] * b.c[n - i];
+        c[n] += y * q;
     }
 }
 
@@ -133,18 +191,23 @@ void logistic_series(long double u0, long double s, long double c[FL_SERIES])
 // replaced by the lower powers of its Chebyshev polynomial T_n(2 x)
 // (Lanczos' economisation), which spreads its size / 2^(n-1) evenly over the
 // cell instead of leaving all of it at the edges.
-void economise(long double c[FL_SERIES])
-{
-    long double T[FL_SERIES][FL_SERIES] = {{0}};   // T_n(2 x), coefficient of x^a
-    T[0][0] = 1.0L;
-    T[1][1] = 2.0L;
-    for (int n = 2; n < FL_SERIES; ++n)
-        for (int a = 0; a <= n; ++a) T[n][a] = (a ? 4.0L * T[n - 1][a - 1] : 0.0L) - T[n - 2][a];
-    for (int n = FL_SERIES - 1; n >= 8; --n) {
-        const long double w = c[n] / T[n][n];
-        for (int a = 0; a <= n; ++a) c[a] -= w * T[n][a];
+struct Economise {
+    long double T[FL_SERIES][FL_SERIES];        // T_n(2 x), coefficient of x^a over that of x^n
+    Economise() : T{{0}}
+    {
+        T[0][0] = 1.0L;
+        T[1][1] = 2.0L;
+        for (int n = 2; n < FL_SERIES; ++n)
+            for (int a = 0; a <= n; ++a) T[n][a] = (a ? 4.0L * T[n - 1][a - 1] : 0.0L) - T[n - 2][a];
+        for (int n = FL_SERIES - 1; n >= 8; --n)
+            for (int a = 0; a <= n; ++a) T[n][a] /= T[n][n];
     }
-}
+    void operator()(long double c[FL_SERIES]) const
+    {
+        for (int n = FL_SERIES - 1; n >= 8; --n)
+            for (int a = n - 2; a >= 0; a -= 2) c[a] -= c[n] * T[n][a];
+    }
+};
 
 // The flutter and power tables of FieldK (formed in long double, stored as
 // double: flutter cells, then power entries).
@@ -154,6 +217,10 @@ void economise(long double c[FL_SERIES])
 // (W below about 3e-3 of a 30 degree sector) keeps the sigmoids.
 // Power entries: spacing 2^-p with the first omitted binomial term below
 // 2^-57, over the map's radii and a quarter of their span on each side.
+// A map pays for them once, but a study of many lattices pays each time: all
+// orders in long double, an exponential for every edge and cell and powl took
+// 6.0 ms for the benchmark's lattice and 43 ms with fringes of a sixth of its
+// sharper one, on the host; this form 1.8 and 7.6 ms with the upload.
 void field_tables(FieldK &k, std::vector<double> &tab)
 {
     double kmax = 0.0;
@@ -173,22 +240,25 @@ void field_tables(FieldK &k, std::vector<double> &tab)
             k.fl_scale = ldexp(1.0, m);
             tab.resize(8 * (size_t)k.fl_n);
             const long double h = ldexpl(1.0L, -m);
+            std::vector<Edge> edges;
+            for (int g = 0; g < k.n_seg; ++g) {      // u at the first cell's middle, h / 2 before the sector
+                const long double ks = k.seg_k[g], mid = -0.5L * h;
+                edges.emplace_back(ks * (mid - (long double)k.seg_x0[g]), ks * h);
+                edges.emplace_back(-ks * (mid - (long double)k.seg_x1[g]), -ks * h);
+            }
+            const Economise economise;
+            Series a, b;
             for (int j = 0; j < k.fl_n; ++j) {
-                const long double mid = ((long double)(j - 1) + 0.5L) * h;
                 long double sum[FL_SERIES] = {0};
+                double high[FL_SERIES] = {0};
                 for (int g = 0; g < k.n_seg; ++g) {
-                    const long double ks = k.seg_k[g];
-                    long double a[FL_SERIES], b[FL_SERIES];
-                    logistic_series(ks * (mid - (long double)k.seg_x0[g]), ks * h, a);
-                    logistic_series(-ks * (mid - (long double)k.seg_x1[g]), -ks * h, b);
-                    for (int n1 = 0; n1 < FL_SERIES; ++n1) {
-                        long double q = 0.0L;
-                        for (int i = 0; i <= n1; ++i) q += a[i] * b[n1 - i];
-                        sum[n1] += (long double)k.seg_y[g] * q;
-                    }
+                    edges[2 * g].at(j, a);
+                    edges[2 * g + 1].at(j, b);
+                    add_product(k.seg_y[g], a, b, sum, high);
                 }
+                for (int n1 = 3; n1 < FL_SERIES; ++n1) sum[n1] = high[n1];
                 economise(sum);
-                for (int a = 0; a < 8; ++a) tab[8 * (size_t)j + a] = (double)sum[a];
+                for (int a1 = 0; a1 < 8; ++a1) tab[8 * (size_t)j + a1] = (double)sum[a1];
             }
         }
     }
@@ -214,7 +284,7 @@ void field_tables(FieldK &k, std::vector<double> &tab)
                 k.pw_c[3] = e * (e - 1) * (e - 2) * (e - 3) / 24;
                 for (int j = 0; j < k.pw_n; ++j) {
                     const long double r = (long double)(k.pw_j0 + j) * (long double)k.pw_h;
-                    tab.push_back((double)((long double)k.B0 * powl(r, (long double)e)));
+                    tab.push_back((double)((long double)k.B0 * expl((long double)e * logl(r))));   // (|e ln r| 2^-64 off)
                     tab.push_back((double)(1.0L / r));
                 }
             }
