@@ -1764,20 +1764,28 @@ cudaError_t launch_pack_nodes(const ffa_field_desc &d, int npad, double *n64, fl
 // so 128 up to 16 warps per SM, 80 while that is one wave, 128 again while that
 // is two, and 80 beyond (order 0, 120 steps, 1e6 particles: 1338 us with 128,
 // 1113 with 80; order 1 1754 and 1486).  Orders 3 and 4 stay at 128 there (order
-// 4, 300000 particles: 830 us, with 80 901; 1e6: 2745 and 2700), and so do the
-// launches that look for crossings, which hold more values over a step.  From order 3 a step's node loads alone need more than 128 (order 4,
-// 10000 particles, 720 steps: 935 us with 128, 791 us with 255).  With space
-// charge the endpoints' registers make 80 spill (60 steps, 1e6 particles: 1898
-// us, 1627 us with 128; 100000: 227 and 224).
+// 4, 300000 particles: 830 us, with 80 901; 1e6: 2745 and 2700).  From order 3 a
+// step's node loads alone need more than 128 (order 4, 10000 particles, 720
+// steps: 935 us with 128, 791 us with 255).
+// Field-error harmonics follow the same rule (order 2, 120 steps: 100000
+// particles 550 us with 128, 358 with 80; 1e6, 30 steps: 966 and 796).
+// With space charge the endpoints' registers make 80 spill: only for the bunches
+// that it keeps in one wave (60 steps, order 2 / 4: 77000 particles 217 / 292 us
+// with 128, 194 / 267 with 80; 113000 231 / 338 and 226 / 314; 1e6 1627 us with
+// 128, 1898 with 80).
+// Launches that look for crossings hold more values over a step and gain from
+// the one wave up to 20 warps per SM (order 2, 120 steps: 90000 particles 473 us
+// with 128, 461 with 80; 100000 480 and 502; 113000 496 and 533), with harmonics
+// up to 24 (113000: 740 and 656).
 static int boris_cap(const PushK &p, bool sc, int max_order)
 {
-    if (sc) return 128;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t warps = (p.n + 31) / 32;
-    if (max_order >= 3 && warps <= (int64_t)8 * sms) return 255;
+    if (!sc && max_order >= 3 && warps <= (int64_t)8 * sms) return 255;
     if (warps <= (int64_t)16 * sms) return 128;
-    if (warps <= (int64_t)24 * sms) return 80;
+    if (warps <= (int64_t)(xing_on(p) && !sc && p.f.n_harm == 0 ? 20 : 24) * sms) return 80;
+    if (sc) return 128;
     return max_order >= 3 || xing_on(p) || warps <= (int64_t)32 * sms ? 128 : 80;
 }
 
@@ -1794,10 +1802,13 @@ static void boris_shaped(const PushK &p, cudaStream_t s, int tb)
 template <int MAXO, bool SC>
 static void boris_launch(const PushK &p, cudaStream_t s, int tb, int)
 {
-    if (p.f.n_harm > 0) return boris_shaped<MAXO, SC, 128, true>(p, s, tb);
     const int cap = boris_cap(p, SC, MAXO);
+    if (p.f.n_harm > 0) {
+        if (cap == 80) return boris_shaped<MAXO, SC, 80, true>(p, s, tb);
+        return boris_shaped<MAXO, SC, 128, true>(p, s, tb);
+    }
+    if (cap == 80) return boris_shaped<MAXO, SC, 80, false>(p, s, tb);
     if constexpr (!SC) {
-        if (cap == 80) return boris_shaped<MAXO, SC, 80, false>(p, s, tb);
         if constexpr (MAXO >= 3) {
             if (cap == 255) return boris_shaped<MAXO, SC, 255, false>(p, s, tb);
         }
