@@ -498,13 +498,19 @@ int ffa_mapgen(const ffa_mapgen_desc *desc, void *stream);
 #define FFA_MLP_WPACK_BYTES 278528   /* bfloat16 copies of W1..W4 for inference */
 #define FFA_MLP_SPLIT_WORK 1048576    /* floats of the training work area beside those per sample */
 
+#define FFA_MLP_STEP_FAILED 0x4D4C502067617665ULL   /* first word of the work area: a step gave up */
+
 /* One optimiser step (no counterpart in the reference, whose tracker has no
  * learned map): forward, mean-squared error over the first n_fit
  * outputs, backward into `grads` (every parameter, same layout), then Adam
  * on the entries whose `mask` byte is non-zero (mask NULL: all) when lr > 0.
  * `step` is the 1-based Adam step (bias correction).  `work` holds
  * 8 * batch * 256 + 24 * batch + FFA_MLP_SPLIT_WORK floats; `loss_part` 148 doubles whose sum is
- * the batch's summed squared error (before the step). */
+ * the batch's summed squared error (before the step).  A step whose bounded
+ * pipeline waits run out marks the first 8 bytes of `work` (from the first
+ * 128-byte boundary in it) with FFA_MLP_STEP_FAILED; its update then writes NaN
+ * to every gradient and to the loss, changes no parameter, moment or counter,
+ * and clears the mark. */
 typedef struct ffa_mlp_train_desc {
     int64_t batch;
     int32_t n_fit;                /* 1..6 */
@@ -535,7 +541,8 @@ int ffa_mlp_gemm(const float *A, int lda, int transA, const float *B, int ldb, i
                  int M, int N, int K, const float *bias, void *stream);
 
 /* Tiles of ffa_mlp_gemm and ffa_mlp_train_step whose bounded pipeline waits
- * ran out since the last call (their outputs, loss or gradients hold NaN);
+ * ran out since the last call (their outputs, or the step's loss and gradients,
+ * hold NaN);
  * reads and clears the device counter, synchronising the device.  No
  * counterpart in the reference (its training path does not exist; the
  * learned map is new). */

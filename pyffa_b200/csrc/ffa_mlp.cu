@@ -1283,11 +1283,20 @@ struct TrainWork {
     float *skip;                // [T][SKIP_SUMS]
     double *loss;               // [2 T]
     int32_t *ticket;
+    // FFA_MLP_STEP_FAILED from a block whose pipeline waits ran out until the
+    // update has seen it: what that block did not write is another step's
+    unsigned long long *failed;
 };
 
 __host__ __device__ inline unsigned char *tile_img(const TrainWork &w, int arr, int64_t t)
 {
     return w.img + ((int64_t)arr * w.T + t) * TT_IMG;
+}
+
+__device__ __forceinline__ void train_gave_up(const TrainWork &w)
+{
+    *w.failed = FFA_MLP_STEP_FAILED;
+    atomicAdd(&g_gemm_timeouts, 1);
 }
 
 __global__ void __launch_bounds__(256) train_pack_kernel(const float *__restrict__ P, TrainWork w)
@@ -1699,8 +1708,6 @@ __global__ void __launch_bounds__(TT_THREADS, 1)
                 if ((et & 3) == 0 && e0 + (et >> 2) < SKIP_SUMS) w.skip[t * SKIP_SUMS + e] = s;
             }
         }
-        if (!ok && u == 2 && lane == 0)                        // gave up: the loss says so
-            for (int64_t t = blockIdx.x; t < w.T; t += gridDim.x) w.loss[2 * t + group] = __longlong_as_double(0x7FF8000000000000ll);
     }
     tc_before_sync();
     __syncthreads();
@@ -1708,7 +1715,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1)
         tc_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
     }
-    if (threadIdx.x == 0 && *abort_flag) atomicAdd(&g_gemm_timeouts, 1);
+    if (threadIdx.x == 0 && *abort_flag) train_gave_up(w);
 }
 
 // Weight gradients.  Blocks 0 .. 8 S - 1: (product, quadrant, split): 128 x 128
@@ -1802,7 +1809,6 @@ __global__ void __launch_bounds__(TG_THREADS, 1) train_wgrad_kernel(TrainWork w)
     }
     __syncthreads();
     tc_after_sync();
-    const bool failed = *abort_flag != 0;
     const int row = 32 * warp + lane;                           // accumulator row
     const uint32_t base = tmem + ((uint32_t)(32 * warp) << 16);
     if (large) {
@@ -1814,8 +1820,6 @@ __global__ void __launch_bounds__(TG_THREADS, 1) train_wgrad_kernel(TrainWork w)
             TMEM_LD32(base + n, v);
             tmem_wait_ld();
             REG_FENCE32(v);
-            if (failed)
-                for (int j = 0; j < 32; ++j) v[j] = 0x7FC00000u;
 #pragma unroll
             for (int j = 0; j < 32; j += 4)
                 out[(int64_t)((n + j) / 4) * H] = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
@@ -1829,7 +1833,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1) train_wgrad_kernel(TrainWork w)
         float *out = w.part16 + ((int64_t)prod * w.SS + split) * (16 * H);
 #pragma unroll
         for (int j = 0; j < 32; ++j)
-            out[(j & 15) * H + 128 * (j >> 4) + row] = __uint_as_float(failed ? 0x7FC00000u : v[j]);
+            out[(j & 15) * H + 128 * (j >> 4) + row] = __uint_as_float(v[j]);
     }
     tc_before_sync();
     __syncthreads();
@@ -1837,7 +1841,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1) train_wgrad_kernel(TrainWork w)
         tc_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128));
     }
-    if (threadIdx.x == 0 && failed) atomicAdd(&g_gemm_timeouts, 1);
+    if (threadIdx.x == 0 && *abort_flag) train_gave_up(w);
 }
 
 struct AdamArgs {
@@ -1849,10 +1853,10 @@ struct AdamArgs {
     int update;
 };
 
-__device__ __forceinline__ void adam_one(const AdamArgs &a, int i, float g, float lr, float c1, float c2)
+__device__ __forceinline__ void adam_one(const AdamArgs &a, int i, float g, float lr, float c1, float c2, bool failed)
 {
-    a.G[i] = g;
-    if (!a.update || (a.mask && !a.mask[i])) return;
+    a.G[i] = failed ? __uint_as_float(0x7FC00000u) : g;
+    if (failed || !a.update || (a.mask && !a.mask[i])) return;
     const float mi = a.b1 * a.m[i] + (1.0f - a.b1) * g;
     const float vi = a.b2 * a.v[i] + (1.0f - a.b2) * g * g;
     a.m[i] = mi;
@@ -1861,6 +1865,7 @@ __device__ __forceinline__ void adam_one(const AdamArgs &a, int i, float g, floa
 }
 
 // Every parameter's gradient from the partial sums, in a fixed order, then Adam.
+// A step that failed gives NaN gradients and loss, and updates nothing.
 // Blocks 0 .. 255: 32 k x 16 n of W2 and W3 (summed along k, which is contiguous
 // in the partial products, updated along n); then 32 parameters a block, the
 // partial sums of each over eight warps; the loss in the last block.
@@ -1871,6 +1876,7 @@ __global__ void __launch_bounds__(256) train_update_kernel(TrainWork w, AdamArgs
 {
     __shared__ float sh[32][33];
     ffa::chain_wait();
+    const bool failed = *w.failed == FFA_MLP_STEP_FAILED;
     float lr = a.lr, c1 = a.c1, c2 = a.c2;
     if (a.lr_table) {
         const int k = *a.counter;
@@ -1899,7 +1905,7 @@ __global__ void __launch_bounds__(256) train_update_kernel(TrainWork w, AdamArgs
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const int k = (tid >> 4) + 16 * j;
-            adam_one(a, base + (k0 + k) * H + n0 + n, sh[k][n] + sh[k][16 + n], lr, c1, c2);
+            adam_one(a, base + (k0 + k) * H + n0 + n, sh[k][n] + sh[k][16 + n], lr, c1, c2, failed);
         }
     } else if (blockIdx.x + 1 < gridDim.x) {
         // parameter r of W1, b1, b2, b3, W4, b4, Ws, bs, Wq: its partial sums
@@ -1948,21 +1954,22 @@ __global__ void __launch_bounds__(256) train_update_kernel(TrainWork w, AdamArgs
         if (wp == 0 && i >= 0) {
             float g = 0.0f;
             for (int k = 0; k < 8; ++k) g += sh[k][lane];
-            adam_one(a, i, g, lr, c1, c2);
+            adam_one(a, i, g, lr, c1, c2, failed);
         }
     } else {
         for (int q = tid; q < 148; q += 256) {
             double s = 0.0;
             for (int64_t z = q; z < 2 * w.T; z += 148) s += w.loss[z];
-            loss_part[q] = s;
+            loss_part[q] = failed ? __longlong_as_double(0x7FF8000000000000ll) : s;
         }
     }
-    // the last block to finish advances the schedule
-    if (a.counter) {
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            if (atomicAdd(w.ticket, 1) == (int)gridDim.x - 1) *a.counter += 1;
+    // the last block to finish advances the schedule and clears the failure
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(w.ticket, 1) == (int)gridDim.x - 1) {
+            if (failed) *w.failed = 0;
+            else if (a.counter) *a.counter += 1;
         }
     }
 }
@@ -1980,6 +1987,7 @@ bool train_layout(TrainWork &w, float *work, int64_t B)
         p += (bytes + 127) & ~int64_t(127);
         return q;
     };
+    w.failed = reinterpret_cast<unsigned long long *>(take(8));
     w.img = take(6 * w.T * TT_IMG);
     w.small = take(2 * w.T * TT_SMALL);
     w.wpk = take(16 * (int64_t)W_CHUNK_BYTES);
