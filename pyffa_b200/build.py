@@ -79,9 +79,11 @@ PROBE_PATH = os.path.join(PKG_DIR, "libffa_probe.so")
 
 
 def build_probe(force: bool = False) -> str:
-    """The benchmark's FP64 peak probe (csrc/probe/ffa_probe.cu)."""
+    """The probe library (csrc/probe/ffa_probe.cu): FMA peaks for the
+    benchmark, the push kernels' reciprocals for their test."""
     src = os.path.join(CSRC, "probe", "ffa_probe.cu")
-    if not force and os.path.exists(PROBE_PATH) and os.path.getmtime(PROBE_PATH) >= os.path.getmtime(src):
+    newest = max(os.path.getmtime(f) for f in (src, os.path.join(CSRC, "ffa_math.cuh")))
+    if not force and os.path.exists(PROBE_PATH) and os.path.getmtime(PROBE_PATH) >= newest:
         return PROBE_PATH
     cmd = [nvcc_path(), *ARCH_FLAGS, "-O3", "-Xcompiler", "-fPIC", "-shared", "-o", PROBE_PATH, src]
     res = subprocess.run(cmd, capture_output=True, text=True)

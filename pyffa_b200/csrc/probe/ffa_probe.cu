@@ -1,8 +1,11 @@
-// ffa_probe.cu -- measurement helper for the benchmark's roofline (not part
-// of the tracking ABI): float64 and float32 FMA throughput kernels giving the
-// FP64 and FP32 pipe peaks of the device they run on.
+// ffa_probe.cu -- measurement helpers (not part of the tracking ABI): float64
+// and float32 FMA throughput kernels giving the FP64 and FP32 pipe peaks of the
+// device they run on, for the benchmark's roofline, and the push kernels'
+// reciprocals element by element, for their test.
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include "../ffa_math.cuh"
 
 __global__ void __launch_bounds__(256) fp64_fma_kernel(double *out, int iters, double a, double b)
 {
@@ -59,5 +62,21 @@ extern "C" int ffa_probe_fp32_fma(int blocks, int iters, float *out, void *strea
     cudaEventElapsedTime(ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+__global__ void reciprocals_kernel(const double *x, double *rs, double *rc, int64_t n)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    rs[i] = ffa::rsqrt64(x[i]);
+    rc[i] = ffa::rcp64(x[i]);
+}
+
+// rs = x^(-1/2), rc = 1 / x (device arrays of n)
+extern "C" int ffa_probe_reciprocals(const double *x, double *rs, double *rc, int64_t n, void *stream)
+{
+    if (n < 1) return 1;
+    reciprocals_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, rs, rc, n);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
