@@ -127,15 +127,19 @@ struct Series {
     bool flat;                          // orders above 0 vanish
 };
 
-void logistic_series(long double c0, long double s, Series &t)
+void logistic_series(long double u0, long double s, Series &t)
 {
-    t.l[0] = c0 < 1e-280L ? 0.0L : c0;  // (the tail's end, clear of denormal numbers)
-    t.flat = t.l[0] == 0.0L || t.l[0] == 1.0L;
-    if (t.flat) return;
+    t.flat = u0 > 46.0L || u0 < -645.0L;                // 1 in long double; the tail's end, clear of denormal numbers
+    if (t.flat) {
+        t.l[0] = u0 > 0.0L ? 1.0L : 0.0L;
+        return;
+    }
+    const long double c0 = 1.0L / (1.0L + expl(-u0));
+    t.l[0] = c0;
     t.l[1] = s * (c0 - c0 * c0);
     t.l[2] = s * (t.l[1] - 2.0L * c0 * t.l[1]) / 2.0L;
     for (int n = 0; n < 3; ++n) t.c[n] = (double)t.l[n];
-    if (c0 < 0x1p-70L) {                // the exponential tail: the products are lost beside c_n
+    if (u0 < -50.0L) {                  // the exponential tail: the products are lost beside c_n
         for (int n = 2; n + 1 < FL_SERIES; ++n) t.c[n + 1] = (double)s * t.c[n] * (1.0 / (n + 1));
         return;
     }
@@ -148,18 +152,6 @@ void logistic_series(long double c0, long double s, Series &t)
         t.c[n + 1] = sd * q * (1.0 / (n + 1));
     }
 }
-
-// One edge of a magnet, cell by cell: sigma of u = u0 + j s.  exp(-u) is carried
-// from cell to cell and formed anew every 16th (16 roundings of 2^-64).
-struct Edge {
-    long double u0, s, step, e;
-    Edge(long double u0_, long double s_) : u0(u0_), s(s_), step(expl(-s_)), e(0.0L) {}
-    void at(int j, Series &t)
-    {
-        e = j & 15 ? e * step : expl(-(u0 + (long double)j * s));
-        logistic_series(1.0L / (1.0L + e), s, t);
-    }
-};
 
 // Adds y a b to the orders l (0 to 2) and c (3 on)
 void add_product(double y, const Series &a, const Series &b, long double l[3], double c[FL_SERIES])
@@ -218,9 +210,9 @@ struct Economise {
 // Power entries: spacing 2^-p with the first omitted binomial term below
 // 2^-57, over the map's radii and a quarter of their span on each side.
 // A map pays for them once, but a study of many lattices pays each time: all
-// orders in long double, an exponential for every edge and cell and powl took
-// 6.0 ms for the benchmark's lattice and 43 ms with fringes of a sixth of its
-// sharper one, on the host; this form 1.8 and 7.6 ms with the upload.
+// orders of every cell in long double took 7.2 ms for the benchmark's
+// lattice and 45 ms with fringes of a sixth of its sharper one, on the host; this
+// form 3.3 and 11 ms with the upload.
 void field_tables(FieldK &k, std::vector<double> &tab)
 {
     double kmax = 0.0;
@@ -240,20 +232,16 @@ void field_tables(FieldK &k, std::vector<double> &tab)
             k.fl_scale = ldexp(1.0, m);
             tab.resize(8 * (size_t)k.fl_n);
             const long double h = ldexpl(1.0L, -m);
-            std::vector<Edge> edges;
-            for (int g = 0; g < k.n_seg; ++g) {      // u at the first cell's middle, h / 2 before the sector
-                const long double ks = k.seg_k[g], mid = -0.5L * h;
-                edges.emplace_back(ks * (mid - (long double)k.seg_x0[g]), ks * h);
-                edges.emplace_back(-ks * (mid - (long double)k.seg_x1[g]), -ks * h);
-            }
             const Economise economise;
             Series a, b;
             for (int j = 0; j < k.fl_n; ++j) {
+                const long double mid = ((long double)(j - 1) + 0.5L) * h;
                 long double sum[FL_SERIES] = {0};
                 double high[FL_SERIES] = {0};
                 for (int g = 0; g < k.n_seg; ++g) {
-                    edges[2 * g].at(j, a);
-                    edges[2 * g + 1].at(j, b);
+                    const long double ks = k.seg_k[g];
+                    logistic_series(ks * (mid - (long double)k.seg_x0[g]), ks * h, a);
+                    logistic_series(-ks * (mid - (long double)k.seg_x1[g]), -ks * h, b);
                     add_product(k.seg_y[g], a, b, sum, high);
                 }
                 for (int n1 = 3; n1 < FL_SERIES; ++n1) sum[n1] = high[n1];
@@ -284,7 +272,7 @@ void field_tables(FieldK &k, std::vector<double> &tab)
                 k.pw_c[3] = e * (e - 1) * (e - 2) * (e - 3) / 24;
                 for (int j = 0; j < k.pw_n; ++j) {
                     const long double r = (long double)(k.pw_j0 + j) * (long double)k.pw_h;
-                    tab.push_back((double)((long double)k.B0 * expl((long double)e * logl(r))));   // (|e ln r| 2^-64 off)
+                    tab.push_back((double)((long double)k.B0 * powl(r, (long double)e)));
                     tab.push_back((double)(1.0L / r));
                 }
             }
@@ -350,7 +338,6 @@ int ffa_fieldmap_create(const ffa_field_desc *d, void *stream, ffa_fieldmap **ou
     k.B0 = d->B0;
     k.k = d->k;
     k.km1 = d->k - 1.0;
-    k.B0k = d->B0 * d->k;
     k.period = 2.0 * PI / (double)d->nsectors;
     k.inv_period = 1.0 / k.period;
     memcpy(k.spoly, d->spoly, sizeof(k.spoly));
