@@ -1385,7 +1385,12 @@ __device__ __forceinline__ void load8(const float *p, float (&v)[8])       // 16
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-// NO: outputs evaluated, 4 (n_fit <= 4) or 6
+// NO: outputs evaluated, 4 (n_fit <= 4) or 6.
+// Of its threads only the weight stream waits for the kernel before
+// (train_pack_kernel, whose packed weights it loads).  The others read what that
+// kernel only reads and write what it does not touch; all that came before the
+// step is complete, because train_pack_kernel is an ordinary launch.  If that one
+// is ever chained too, every thread here has to wait.
 template <int NO>
 __global__ void __launch_bounds__(TT_THREADS, 1)
     train_tile_kernel(const float *__restrict__ P, const float *__restrict__ X, const float *__restrict__ Y, TrainWork w,

@@ -24,8 +24,12 @@
 // sin/cos pairs per step and is the more accurate of the two.  Particles that
 // are skipped (not injected or lost) take the reference's exact Cartesian
 // round trip, which perturbs r, vr and dfi/dt by rounding every step.
-// Expressions otherwise keep the reference's evaluation order; the compiler may
-// fuse a multiply and an add into one FMA (at most an ulp per operation).
+// The float64 kernels form the reference's values, not its expressions: the
+// mid-plane field from tables, divisions and square roots from ffa_math.cuh, the
+// momentum (Boris) and what depends on the energy (RK4) carried from step to
+// step.  Each differs from the reference's expression by about an ulp.  The FP32C
+// kernels and the rare branches keep its evaluation order; the compiler may fuse
+// a multiply and an add into one FMA (at most an ulp per operation).
 #include <float.h>
 
 #include "ffa_internal.cuh"
@@ -92,16 +96,6 @@ __device__ __noinline__ double2 flutter_direct(const FieldK &f, double fs)
 // B0 r^(k-1) for radii outside the power table
 __device__ __noinline__ double power_direct(const FieldK &f, double r) { return f.B0 * exp(f.km1 * log(r)); }
 
-// The mid-plane field and its z-linear terms.  Both one-dimensional factors
-// come from tables made with the map (fl_tab and pw_tab of FieldK): the flutter sum as degree-7 polynomials over cells of 2^-m rad,
-// B0 r^(k-1) as a five-term binomial series about the nearest multiple of
-// 2^-p m.  The cell coordinates are exact (power-of-two cells), so the
-// evaluation adds a few ulp, as the exponentials and the 16-term series about
-// the map centre did before; without their branches and divisions the field is
-// one stretch of code whose chains overlap.  It is bound by dependent FP64
-// latency and issue.  Measured (720 steps, z-Taylor order 2, RF): 1e5
-// particles Boris 2.47 -> 2.07 ms, RK4 11.3 -> 9.6 ms; 1e4 particles, order 4:
-// 1.87 -> 1.74 ms; 1280 azimuth-domain tracks of 523 steps: 2.46 -> 1.59 ms.
 // One flutter cell and the position in it
 struct FlutterCell {
     double c[8], x;
@@ -531,8 +525,8 @@ __device__ __forceinline__ void status_add(int64_t *status, int lost, int bad, i
 // Azimuth-crossing test of detect_azimuth_crossing (src/FFAG_MathTools.py:
 // 1633-1695) on the step's pre / post azimuth, and the record append.  The
 // reductions mod 2 pi are a - 2 pi floor(a / 2 pi) with no fused multiply-add,
-// as in fast_mod_parallel (src/FFAG_MathTools.py:1554-1557); the target comes
-// targets come in already reduced to [0, 2 pi).
+// as in fast_mod_parallel (src/FFAG_MathTools.py:1554-1557); the targets come in
+// already reduced to [0, 2 pi).
 __device__ __forceinline__ double mod_2pi(double a)
 {
     const double tw = 2.0 * PI;
@@ -773,7 +767,7 @@ __device__ __forceinline__ void field_mixed(const FieldK &f, double r, double ir
         B0r = f.c1 * g * r;
     }
     double fs = fim;
-    if (!f.spiral_zero) {   // as in analytic_b64
+    if (!f.spiral_zero) {   // as in tables_fetch
         fs = fim - spiral;
         fs -= f.period * floor(fs * f.inv_period);
     }
@@ -1181,7 +1175,7 @@ __device__ __forceinline__ void field_f32(const FieldK &f, double r, double fim,
     }
     float spiral_p = 0.0f;
     double fs = fim;
-    if (!f.spiral_zero) {   // as in analytic_b64, in float64 (spiral lattices only)
+    if (!f.spiral_zero) {   // as in tables_fetch, in float64 (spiral lattices only)
         double spiral = 0.0, sp = 0.0;
         for (int a = 0; a < f.n_spoly; ++a) spiral = spiral * r + f.spoly[a];
         for (int a = 0; a < f.n_spolyp; ++a) sp = sp * r + f.spolyp[a];
