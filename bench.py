@@ -33,19 +33,22 @@ N_PARTICLES = 100_000
 STEPS_PER_TURN = 720
 REF_SAMPLE_STEPS = 72       # steps of a turn the reference arm runs per step
 MAX_ORDER = 2
-# algorithmic float64 operations per particle-step of one Boris step: the
+# float64 operations per particle-step of one Boris step evaluated directly: the
 # arithmetic of the reference's step (field, RF kick, Cartesian round trip,
-# Boris push; transcendentals not counted), the roofline's numerator
+# Boris push; transcendentals not counted).  The roofline's numerator, kept so that
+# lines compare over time; the kernel's tables do the field with fewer
 FP64_FLOP_PER_PARTICLE_STEP = 300.0
 # the kernel's executed float64 operations per particle-step (2 per DFMA, 1
 # per DADD / DMUL), counted by ncu on this workload: reported beside it
 FP64_EXEC_FLOP_PER_PARTICLE_STEP = 213.7
-# algorithmic float64 operations per particle-step of one RK4 step: four
+# the same of one RK4 step evaluated directly: four
 # right-hand sides (azimuth mod sector 3, analytic field 93, z-Taylor sum 77,
 # RF window test 4, equations of motion 40) and the stage arithmetic (k = h d,
 # the stage states and the weighted sum, seven components each: 112), i.e.
 # 4 x 217 + 112
 RK4_FLOP_PER_PARTICLE_STEP = 980.0
+# and executed by its kernel (ncu)
+RK4_EXEC_FLOP_PER_PARTICLE_STEP = 774.0
 # DRAM bytes (read + write) of one launch (one turn, 1e5 particles) from an
 # ncu capture of the same launch, L2 flushed before it
 BORIS_TRAFFIC_PER_LAUNCH = 17.443e6
@@ -1044,7 +1047,7 @@ def main():
         ach = FP64_FLOP_PER_PARTICLE_STEP * pstep / avg_launch_s / 1e12
         ach_x = FP64_EXEC_FLOP_PER_PARTICLE_STEP * pstep / avg_launch_s / 1e12
         roof.update({"achieved": ach, "frac": ach / peak64,
-                     "flop_per_particle_step": FP64_FLOP_PER_PARTICLE_STEP, "flop_basis": "algorithmic",
+                     "flop_per_particle_step": FP64_FLOP_PER_PARTICLE_STEP, "flop_basis": "direct evaluation",
                      "executed": {"flop_per_particle_step": FP64_EXEC_FLOP_PER_PARTICLE_STEP,
                                   "achieved": ach_x, "frac": ach_x / peak64}})
         hbm_peak = None
@@ -1075,7 +1078,10 @@ def main():
             ach = RK4_FLOP_PER_PARTICLE_STEP * N_PARTICLES * STEPS_PER_TURN / (rk4["ms_per_turn"] * 1e-3) / 1e12
             rk4["roofline"] = {"bound": "fp64", "achieved": ach, "peak": peak64, "unit": "TFLOP/s",
                                "frac": ach / peak64, "flop_per_particle_step": RK4_FLOP_PER_PARTICLE_STEP,
-                               "flop_basis": "algorithmic",
+                               "flop_basis": "direct evaluation",
+                               "executed": {"flop_per_particle_step": RK4_EXEC_FLOP_PER_PARTICLE_STEP,
+                                            "frac": ach / peak64 * RK4_EXEC_FLOP_PER_PARTICLE_STEP /
+                                            RK4_FLOP_PER_PARTICLE_STEP},
                                "peak_source": "measured live: float64 FMA probe kernel (libffa_probe.so)"}
         acc = None
         if not args.no_accuracy and solo:
