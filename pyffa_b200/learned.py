@@ -578,6 +578,7 @@ def train(params, X, T, epochs=10, batch=8192, lr=2e-3, lr_min=1e-5, warmup=200,
     end (exactly: a power of two).  graph: the learning-rate schedule as a
     device table and every step after the first a replay of one captured
     CUDA graph (Trainer.graph_step); else one host-scheduled call per step.
+    A step of a replayed run that gave up (it updates nothing) raises at the end.
     Returns the history [(step, mse)] of the scaled problem (sampled when
     log_every > 0) and the trainer."""
     torch = _torch()
@@ -621,6 +622,8 @@ def train(params, X, T, epochs=10, batch=8192, lr=2e-3, lr_min=1e-5, warmup=200,
     if sigma != 1.0:
         block(params, "W4").mul_(sigma)
         block(params, "b4").mul_(sigma)
+    if graph and int(tr.counter.item()) != k:      # the device counts the steps that updated
+        raise RuntimeError(f"{k - int(tr.counter.item())} of {k} training steps gave up (ffa_mlp_gemm_timeouts)")
     return hist, tr
 
 

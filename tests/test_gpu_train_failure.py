@@ -62,3 +62,28 @@ def test_failed_step_updates_nothing(B, mode):
         assert torch.equal(v, w)
     if lr is not None:
         assert int(a.counter) == int(b.counter) == 3
+
+
+@pytest.mark.parametrize("fail", [False, True])
+def test_training_run_reports_it(fail, monkeypatch):
+    from pyffa_b200 import learned
+    rng = np.random.default_rng(1)
+    X = np.zeros((4096, 8), np.float32)
+    X[:, :5] = rng.uniform(-1, 1, (4096, 5))
+    X = torch.from_numpy(X).cuda()
+    T = X + 0.05 * torch.sin(3 * X)
+    plain, calls = learned.Trainer.graph_step, []
+
+    def graph_step(tr, x, t):
+        calls.append(1)
+        if fail and len(calls) == 3:
+            mark(tr)
+        plain(tr, x, t)
+    monkeypatch.setattr(learned.Trainer, "graph_step", graph_step)
+    p = torch.from_numpy(learned.init_params(0)).cuda()
+    if fail:
+        with pytest.raises(RuntimeError, match="1 of 8 training steps gave up"):
+            learned.train(p, X, T, epochs=2, batch=1024)
+    else:
+        learned.train(p, X, T, epochs=2, batch=1024)
+    assert bool(torch.isfinite(p).all())
